@@ -18,6 +18,7 @@
 #include "kernels.cuh"
 
 #include <algorithm>
+#include <cmath>
 #include <cstdio>
 #include <cstring>
 #include <mutex>
@@ -64,7 +65,7 @@ enum OpType : uint32_t { OP_COPY = 0, OP_CLUT = 1, OP_PASS = 2, OP_SNAPSHOT = 3 
 
 struct PassOp
 {
-	size_t pos_off, attr_off, prim_off, states_off, textures_off, images_off;
+	size_t pos_off, attr_off, prim_off, states_off, textures_off, images_off, samplers_off;
 	uint32_t num_texels, max_texels, max_levels;
 	uint32_t num_prims, num_states, num_textures;
 	uint32_t tile_size_log2, has_aa1, has_scanmsk, has_mipmap, has_ss_textures;
@@ -221,6 +222,23 @@ static void build_phase_lut(uint32_t rx, uint32_t ry, uint32_t *lut)
 			candidates(2 * x, 2 * y, pts_nearest, 0, c);
 			lut[G * G * 2 + y * (G / 2) + x] = uint32_t(c[0].sample);
 		}
+}
+
+// Level 0 sampling constants of one axis (TexAxis): `mode` keeps only the
+// region wrap modes, plain REPEAT and CLAMP come from the primitive's bit.
+static TexAxis sampler_axis(uint32_t mode, bool clamp, uint32_t size_log2, uint32_t lo, uint32_t hi, uint32_t place)
+{
+	if (mode < WRAP_REGION_CLAMP)
+		mode = clamp ? WRAP_CLAMP : WRAP_REPEAT;
+	const WrapAxis w = wrap_axis(mode, size_log2, lo, hi);
+	TexAxis a = { w.and_mask, w.or_mask, w.lo, w.hi, -INFINITY, INFINITY, 16.0f * float(1u << size_log2), place };
+	if (clamp)
+	{
+		const bool region = mode == WRAP_REGION_CLAMP;
+		a.clamp_lo = 16.0f * (float(region ? lo : 0u) + 0.5f);
+		a.clamp_hi = 16.0f * (float(region ? hi : (1u << size_log2) - 1u) + 0.5f);
+	}
+	return a;
 }
 
 struct CudaBackend
@@ -687,9 +705,11 @@ struct CudaBackend
 		size_t st_bytes = size_t(std::max<uint32_t>(rp->num_states, 1)) * sizeof(pgs_state_vector);
 		size_t tex_bytes = size_t(std::max<uint32_t>(rp->num_textures, 1)) * sizeof(pgs_texture_desc);
 		size_t img_bytes = size_t(std::max<uint32_t>(rp->num_textures, 1)) * TEX_SLOTS * sizeof(TexImage);
+		size_t smp_bytes = size_t(std::max<uint32_t>(rp->num_textures, 1)) * sizeof(TexSampler);
 		size_t base;
 		size_t total = align_up(pos_bytes, 256) + align_up(attr_bytes, 256) + align_up(prim_bytes, 256) +
-		               align_up(st_bytes, 256) + align_up(tex_bytes, 256) + align_up(img_bytes, 256);
+		               align_up(st_bytes, 256) + align_up(tex_bytes, 256) + align_up(img_bytes, 256) +
+		               align_up(smp_bytes, 256);
 		int r = arena_alloc(total, base);
 		if (r)
 			return r;
@@ -723,11 +743,14 @@ struct CudaBackend
 		if (rp->num_textures)
 			memcpy(h_arena + p.textures_off, rp->textures, rp->num_textures * sizeof(pgs_texture_desc));
 		p.images_off = p.textures_off + align_up(tex_bytes, 256);
+		p.samplers_off = p.images_off + align_up(img_bytes, 256);
 		{
 			// Decoded extent of each mip level covers every texel index the wrap
 			// modes can produce at that level (region bounds scale with the level).
 			TexImage *im = reinterpret_cast<TexImage *>(h_arena + p.images_off);
+			TexSampler *smp = reinterpret_cast<TexSampler *>(h_arena + p.samplers_off);
 			memset(im, 0, img_bytes);
+			memset(smp, 0, smp_bytes);
 			uint64_t texels = 0;
 			uint32_t max_texels = 0, max_levels = 1;
 			for (uint32_t i = 0; i < rp->num_textures; i++)
@@ -762,6 +785,12 @@ struct CudaBackend
 					uint32_t n = m.ext_u * m.ext_v;
 					texels += n;
 					max_texels = std::max(max_texels, n);
+				}
+				const TexImage &base_image = im[i * TEX_SLOTS];
+				for (uint32_t clamp = 0; clamp < 2; clamp++)
+				{
+					smp[i].u[clamp] = sampler_axis(t.wms, clamp, t.tw_log2, t.minu, t.maxu, base_image.offset);
+					smp[i].v[clamp] = sampler_axis(t.wmt, clamp, t.th_log2, t.minv, t.maxv, base_image.ext_u);
 				}
 			}
 			if (texels > (uint64_t(1) << 31))
@@ -1493,6 +1522,7 @@ struct CudaBackend
 		P.states = reinterpret_cast<const pgs_state_vector *>(d_arena + p.states_off);
 		P.textures = reinterpret_cast<const pgs_texture_desc *>(d_arena + p.textures_off);
 		P.tex_images = reinterpret_cast<const TexImage *>(d_arena + p.images_off);
+		P.samplers = reinterpret_cast<const TexSampler *>(d_arena + p.samplers_off);
 		P.max_tex_levels = p.max_levels;
 		P.rp_is_blur_mask = p.rp_is_blur_mask;
 		P.force_linear_ss = 0;
