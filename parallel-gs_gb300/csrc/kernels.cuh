@@ -209,16 +209,25 @@ constexpr uint32_t ERROR_FLAG_TILE_OVERFLOW = 1u << 0;
 
 __constant__ uint8_t c_rcp_tab[256];
 
-// Occupancy target of the shading kernels in 256-thread units per SM: 4 means
-// at most 64 registers per thread for the 1x..4x variants.  The plain 4x
-// variant (no AA1, no mipmaps) asks for 5 CTAs (48 registers, a few spills):
-// measured on the C2 frame, 3 CTAs 1.24 ms, 4 CTAs 1.10 ms, 5 CTAs 1.09 ms.
-// The AA1 / mipmap variants, larger, stay at 4.
+// Largest shading CTA, as the sampling rate it holds a whole sub-tile of, and
+// occupancy targets of the shading kernels in 256-thread units per SM: 4 means
+// at most 64 registers per thread.  Up to 4x the walk is bound by issue and
+// spills cost more than warps bring (textured 4x frame, 52,000 primitives: 4 CTAs
+// 618 us, 5 631 us, 6 642 us).  The plain variants (no AA1, no mipmaps) at 8x
+// and 16x wait on loads with few primitives per sub-tile (feedback frame, 100,000
+// primitives in ten passes, at 16x: 4 CTAs 4.02 ms, 5 3.79 ms, 6 3.66 ms).  CTA
+// size on the same frame at 16x: 128 threads 3.91 ms, 256 3.79 ms, 512 4.22 ms.
+#ifndef PGS_SHADE_CTA_NS
+#define PGS_SHADE_CTA_NS 4
+#endif
 #ifndef PGS_SHADE_OCC
 #define PGS_SHADE_OCC 4
 #endif
+#ifndef PGS_SHADE_OCC_HIGH_RATE
+#define PGS_SHADE_OCC_HIGH_RATE 6
+#endif
 #define PGS_SHADE_MIN_BLOCKS(NS, LARGE) \
-	((NS) == 4 && !(LARGE) ? PGS_SHADE_OCC + 1 : (PGS_SHADE_OCC * 4 / (NS) > 0 ? PGS_SHADE_OCC * 4 / (NS) : 1))
+	(((NS) >= 8 && !(LARGE) ? PGS_SHADE_OCC_HIGH_RATE : PGS_SHADE_OCC) * 4 / ((NS) < PGS_SHADE_CTA_NS ? (NS) : PGS_SHADE_CTA_NS))
 
 // ---------------------------------------------------------------------------
 // Scalar helpers.
@@ -2549,28 +2558,96 @@ __device__ __forceinline__ void walk_batch(const ShadeCtx &C, const uint32_t *id
 	}
 }
 
+// Threads of a shading CTA: the 64 * NS samples of a sub-tile, in CTAs of 256 at
+// most.  The CTAs of a sub-tile expand its list each for themselves, which is
+// cheap next to what whole-sub-tile CTAs of 512 and 1024 threads cost at 8x and
+// 16x, two and one of them per SM, waiting for each other at every barrier:
+// feedback frame of 100,000 primitives, 8x 2.48 -> 2.07 ms, 16x 5.07 -> 3.66 ms.
+template <int NS>
+struct ShadeCta
+{
+	static constexpr uint32_t THREADS = NS < PGS_SHADE_CTA_NS ? 64u * NS : 64u * PGS_SHADE_CTA_NS;
+	static constexpr uint32_t PARTS = 64u * NS / THREADS; // CTAs per sub-tile
+	static constexpr uint32_t WARPS = THREADS / 32u;
+};
+
 // The sub-tile's primitive list, expanded by the whole CTA into primitive
 // indices in ascending order in shared memory (CAP at a time), then walked by
-// each warp on its own, 32 primitives at a time: every lane tests one
-// primitive against the warp's rectangle and the warp shades, in order, the
-// primitives that can touch it.  The primitives a warp skips are the ones
-// whose coverage test would fail on every lane, so each warp sees the same
-// sequence of covering primitives as walking the whole list.  Expansion:
-// each warp counts the primitives under its summary words, warp 0 turns the
-// counts into offsets, and each warp writes its indices at those offsets.
+// each warp on its own, 32 primitives at a time.  Expansion: each warp counts
+// the primitives under its summary words, every warp turns the counts into
+// offsets, and each writes the indices under its words at those offsets.
+constexpr uint32_t LIST_CAP = 2048u;
+// One summary word per 32 mask words of 32 primitives.
+constexpr uint32_t LIST_MAX_SW = (PGS_MAX_PRIMITIVES_PER_FLUSH + 1023u) / 1024u;
+static_assert(LIST_MAX_SW <= 64, "list_scan holds two offsets per lane");
+
+struct ListShared
+{
+	uint32_t ids[LIST_CAP];
+	uint32_t count[LIST_MAX_SW];
+};
+
+// Offsets of summary words `lane` and `lane + 32` in the list, and its length.
+struct ListScan
+{
+	uint32_t lo, hi, total;
+};
+
+__device__ __forceinline__ uint32_t warp_scan(uint32_t v, uint32_t lane)
+{
+	uint32_t x = v;
+	#pragma unroll
+	for (int o = 1; o < 32; o <<= 1)
+	{
+		const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+		if (lane >= uint32_t(o))
+			x += y;
+	}
+	return x;
+}
+
+template <uint32_t WARPS>
+__device__ __forceinline__ ListScan list_scan(const DevInstance &I, const uint32_t *summary, const uint32_t *mask, ListShared &L)
+{
+	const unsigned full = 0xffffffffu;
+	const uint32_t lane = threadIdx.x & 31u, SW = I.summary_words;
+	for (uint32_t sw = threadIdx.x >> 5; sw < SW; sw += WARPS)
+	{
+		const uint32_t words = __ldg(summary + sw);
+		const uint32_t mw = ((words >> lane) & 1u) ? __ldg(mask + sw * 32u + lane) : 0u;
+		const uint32_t c = __reduce_add_sync(full, uint32_t(__popc(mw)));
+		if (lane == 0)
+			L.count[sw] = c;
+	}
+	__syncthreads();
+	ListScan r;
+	const uint32_t v = lane < SW ? L.count[lane] : 0u, x = warp_scan(v, lane);
+	r.lo = x - v;
+	r.total = __shfl_sync(full, x, 31);
+	r.hi = 0;
+	if (SW > 32u)
+	{
+		const uint32_t w = lane + 32u < SW ? L.count[lane + 32u] : 0u, y = warp_scan(w, lane);
+		r.hi = r.total + y - w;
+		r.total += __shfl_sync(full, y, 31);
+	}
+	return r;
+}
+
+// Walks the list: without AA1 through coverage masks (walk_batch); with AA1
+// every lane tests one primitive against the warp's rectangle (may_cover) and
+// the warp shades, in order, the primitives that can touch it, so that it sees
+// the same sequence of covering primitives as walking the whole list.
 template <int NS, bool SS, bool AA, bool MIP>
 __device__ __forceinline__ void walk_culled(const ShadeCtx &C, const DevInstance &I, const uint32_t *summary,
-                                            const uint32_t *mask, uint32_t t, SampleState &S, uint32_t &covered)
+                                            const uint32_t *mask, const ListScan &scan, ListShared &L, uint32_t t,
+                                            SampleState &S, uint32_t &covered)
 {
-	constexpr uint32_t T = 64u * NS, WARPS = T / 32u, CAP = 2048u;
-	// One summary word per 32 mask words of 32 primitives.
-	constexpr uint32_t MAX_SW = (PGS_MAX_PRIMITIVES_PER_FLUSH + 1023u) / 1024u;
-	__shared__ uint32_t s_ids[CAP];
-	__shared__ uint32_t s_off[MAX_SW + 1];
+	constexpr uint32_t WARPS = ShadeCta<NS>::WARPS;
 	__shared__ int4 s_rect[AA ? WARPS : 1];
 	__shared__ int2 s_smp[NS];
 	const PassParams &P = *C.P;
-	const uint32_t lane = t & 31u, warp = t >> 5;
+	const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
 	const unsigned full = 0xffffffffu;
 	const uint32_t SW = I.summary_words;
 	WarpPlace W;
@@ -2583,8 +2660,8 @@ __device__ __forceinline__ void walk_culled(const ShadeCtx &C, const DevInstance
 		W.py0 = __shfl_sync(full, py, 0);
 		W.smp = s_smp;
 		my_bit = B::bit(t % NS, uint32_t(px - W.px0), uint32_t(py - W.py0));
-		if (t < NS)
-			s_smp[t] = make_int2((S.hx - (px << C.dim)) << (3 - C.dim), (S.hy - (py << C.dim)) << (3 - C.dim));
+		if (threadIdx.x < NS)
+			s_smp[threadIdx.x] = make_int2((S.hx - (px << C.dim)) << (3 - C.dim), (S.hy - (py << C.dim)) << (3 - C.dim));
 		if (P.has_scanmsk)
 		{
 			even_rows = __reduce_or_sync(full, (S.hy & 1) ? 0u : 1u << my_bit);
@@ -2599,69 +2676,29 @@ __device__ __forceinline__ void walk_culled(const ShadeCtx &C, const DevInstance
 		if (lane == 0)
 			s_rect[warp] = r;
 	}
-	for (uint32_t sw = warp; sw < SW; sw += WARPS)
-	{
-		const uint32_t words = __ldg(summary + sw);
-		const uint32_t mw = ((words >> lane) & 1u) ? __ldg(mask + sw * 32u + lane) : 0u;
-		const uint32_t c = __reduce_add_sync(full, uint32_t(__popc(mw)));
-		if (lane == 0)
-			s_off[sw] = c;
-	}
-	__syncthreads();
-	if (warp == 0)
-	{
-		uint32_t carry = 0;
-		for (uint32_t base = 0; base < SW; base += 32u)
-		{
-			const uint32_t i = base + lane;
-			const uint32_t v = i < SW ? s_off[i] : 0u;
-			uint32_t x = v;
-			#pragma unroll
-			for (int o = 1; o < 32; o <<= 1)
-			{
-				const uint32_t y = __shfl_up_sync(full, x, o);
-				if (lane >= uint32_t(o))
-					x += y;
-			}
-			if (i < SW)
-				s_off[i] = carry + x - v;
-			carry += __shfl_sync(full, x, 31);
-		}
-		if (lane == 0)
-			s_off[SW] = carry;
-	}
-	__syncthreads();
-	const uint32_t total = s_off[SW];
-	for (uint32_t round = 0; round < total; round += CAP)
+	const uint32_t total = scan.total;
+	for (uint32_t round = 0; round < total; round += LIST_CAP)
 	{
 		for (uint32_t sw = warp; sw < SW; sw += WARPS)
 		{
-			const uint32_t off = s_off[sw], end = s_off[sw + 1];
-			if (end <= round || off >= round + CAP)
+			const uint32_t off = __shfl_sync(full, sw < 32u ? scan.lo : scan.hi, int(sw & 31u)), count = L.count[sw];
+			if (!count || off + count <= round || off >= round + LIST_CAP)
 				continue;
 			const uint32_t words = __ldg(summary + sw);
 			const uint32_t mw = ((words >> lane) & 1u) ? __ldg(mask + sw * 32u + lane) : 0u;
 			const uint32_t pc = uint32_t(__popc(mw));
-			uint32_t x = pc;
-			#pragma unroll
-			for (int o = 1; o < 32; o <<= 1)
-			{
-				const uint32_t y = __shfl_up_sync(full, x, o);
-				if (lane >= uint32_t(o))
-					x += y;
-			}
-			uint32_t pos = off + x - pc;
+			uint32_t pos = off + warp_scan(pc, lane) - pc;
 			const uint32_t prim_base = I.prim_lo + (sw * 32u + lane) * 32u;
 			for (uint32_t m = mw; m; m &= m - 1u, pos++)
-				if (pos >= round && pos < round + CAP)
-					s_ids[pos - round] = prim_base + uint32_t(__ffs(m) - 1);
+				if (pos >= round && pos < round + LIST_CAP)
+					L.ids[pos - round] = prim_base + uint32_t(__ffs(m) - 1);
 		}
 		__syncthreads();
-		const uint32_t n = min(total - round, CAP);
+		const uint32_t n = min(total - round, LIST_CAP);
 		if constexpr (!AA)
 		{
 			for (uint32_t kb = 0; kb < n; kb += 32u)
-				walk_batch<NS, SS>(C, s_ids + kb, min(n - kb, 32u), W, my_bit, even_rows, even_pixels, round + kb + 32u >= total, S,
+				walk_batch<NS, SS>(C, L.ids + kb, min(n - kb, 32u), W, my_bit, even_rows, even_pixels, round + kb + 32u >= total, S,
 				                   covered);
 		}
 		else
@@ -2672,7 +2709,7 @@ __device__ __forceinline__ void walk_culled(const ShadeCtx &C, const DevInstance
 			bool hit = false;
 			if (k < n)
 			{
-				pi = s_ids[k];
+				pi = L.ids[k];
 				hit = may_cover<AA>(P.setup[pi], P.prims[pi].state, s_rect[warp], C.dim);
 			}
 			uint32_t bits = __ballot_sync(full, hit);
@@ -2683,7 +2720,7 @@ __device__ __forceinline__ void walk_culled(const ShadeCtx &C, const DevInstance
 				process_primitive<SS, AA, MIP>(C, __shfl_sync(full, pi, b), S, covered);
 			}
 		}
-		if (round + CAP < total)
+		if (round + LIST_CAP < total)
 			__syncthreads();
 	}
 }
@@ -2715,11 +2752,21 @@ __device__ __forceinline__ uint32_t subtile_mode(const PassParams &P, const DevI
 // the sub-tile's primitive bitmask on its own and needs no barrier.
 template <int NS, bool SS, bool AA, bool MIP = false, bool CULL = false>
 __device__ __forceinline__ void shade_subtile(const PassParams &P, const DevInstance &I, const uint32_t *sub_masks,
-                                              const uint32_t *sub_summary, uint32_t sub, uint32_t t)
+                                              const uint32_t *sub_summary, uint32_t sub, uint32_t t, ListShared *list = nullptr)
 {
 	const uint32_t gx = sub % I.sub_w, gy = sub / I.sub_w;
 	const uint32_t *summary = sub_summary + size_t(sub) * I.summary_words;
 	const uint32_t *mask = sub_masks + size_t(sub) * I.mask_words;
+
+	// The list first: most sub-tiles of a pass of small primitives have none,
+	// and the samples' loads overlap its expansion.
+	ListScan scan = {};
+	if constexpr (CULL)
+	{
+		scan = list_scan<ShadeCta<NS>::WARPS>(I, summary, mask, *list);
+		if (!scan.total)
+			return;
+	}
 
 	ShadeCtx C;
 	C.P = &P;
@@ -2811,7 +2858,7 @@ __device__ __forceinline__ void shade_subtile(const PassParams &P, const DevInst
 	// Walk the primitive list in ascending order: summary word -> mask words -> bits.
 	uint32_t covered = 0;
 	if constexpr (CULL)
-		walk_culled<NS, SS, AA, MIP>(C, I, summary, mask, t, S, covered);
+		walk_culled<NS, SS, AA, MIP>(C, I, summary, mask, scan, *list, t, S, covered);
 	else
 	for (uint32_t sbase = 0; sbase < I.summary_words; sbase += 32u)
 	{
@@ -2846,16 +2893,15 @@ __device__ __forceinline__ void shade_subtile(const PassParams &P, const DevInst
 
 	// Covered-sample counter: one atomic per warp.
 	{
-		uint32_t c = covered;
-		#pragma unroll
-		for (int o = 16; o >= 1; o >>= 1)
-			c += __shfl_xor_sync(0xffffffffu, c, o);
+		const uint32_t c = __reduce_add_sync(0xffffffffu, covered);
 		if (lane == 0 && c)
 			atomicAdd(P.fragment_counter, (unsigned long long)c);
 	}
 
 	// end_tile
 	const unsigned full = 0xffffffffu;
+	if (!__any_sync(full, S.color_dirty || S.depth_dirty))
+		return;
 	uint32_t group_lane0 = (t & 31u) & ~uint32_t(NS - 1);
 	bool req_color = false, req_depth = false;
 	bool color_dirty = S.color_dirty, depth_dirty = S.depth_dirty;
@@ -2957,15 +3003,17 @@ __device__ __forceinline__ void shade_subtile(const PassParams &P, const DevInst
 }
 
 template <int NS, bool SS, bool AA, bool MIP>
-__global__ void __launch_bounds__(64 * NS, PGS_SHADE_MIN_BLOCKS(NS, AA || MIP)) shade_kernel(PassParams P, DevInstance I, const uint32_t *sub_masks,
+__global__ void __launch_bounds__(ShadeCta<NS>::THREADS, PGS_SHADE_MIN_BLOCKS(NS, AA || MIP)) shade_kernel(PassParams P, DevInstance I, const uint32_t *sub_masks,
                                                         const uint32_t *sub_summary, const uint32_t *tile_flags)
 {
-	const uint32_t sub = blockIdx.x;
+	constexpr uint32_t PARTS = ShadeCta<NS>::PARTS;
+	__shared__ ListShared list;
+	const uint32_t sub = blockIdx.x / PARTS, part = blockIdx.x % PARTS;
 	if (sub >= I.sub_w * I.sub_h)
 		return;
 	if (subtile_mode(P, I, tile_flags, sub) != (SS ? 2u : 1u))
 		return;
-	shade_subtile<NS, SS, AA, MIP, true>(P, I, sub_masks, sub_summary, sub, threadIdx.x);
+	shade_subtile<NS, SS, AA, MIP, true>(P, I, sub_masks, sub_summary, sub, part * ShadeCta<NS>::THREADS + threadIdx.x, &list);
 }
 
 // ---------------------------------------------------------------------------
