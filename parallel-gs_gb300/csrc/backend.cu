@@ -286,8 +286,6 @@ struct CudaBackend
 	uint8_t *d_heuristic_action = nullptr;
 	uint32_t *d_masks = nullptr;
 	size_t masks_cap = 0;
-	uint32_t *d_flags = nullptr;
-	size_t flags_cap = 0;
 	uint32_t *d_texels = nullptr;
 	size_t texels_cap = 0;
 	uint32_t *d_circuit = nullptr;
@@ -525,7 +523,6 @@ struct CudaBackend
 		cudaFree(d_heuristic);
 		cudaFree(d_heuristic_action);
 		cudaFree(d_masks);
-		cudaFree(d_flags);
 		cudaFree(d_texels);
 		cudaFree(d_circuit);
 		cudaFree(d_readback);
@@ -1049,7 +1046,7 @@ struct CudaBackend
 		return r;
 	}
 
-	int ensure_masks(size_t words, size_t tiles)
+	int ensure_masks(size_t words)
 	{
 		if (words > masks_cap)
 		{
@@ -1057,14 +1054,6 @@ struct CudaBackend
 			size_t cap = std::max(words, masks_cap * 2);
 			CUDA_TRY(cudaMalloc(&d_masks, cap * sizeof(uint32_t)));
 			masks_cap = cap;
-			if (graph_exec) { cudaGraphExecDestroy(graph_exec); graph_exec = nullptr; }
-		}
-		if (tiles > flags_cap)
-		{
-			cudaFree(d_flags);
-			size_t cap = std::max(tiles, flags_cap * 2);
-			CUDA_TRY(cudaMalloc(&d_flags, cap * sizeof(uint32_t)));
-			flags_cap = cap;
 			if (graph_exec) { cudaGraphExecDestroy(graph_exec); graph_exec = nullptr; }
 		}
 		return PGS_OK;
@@ -1093,7 +1082,7 @@ struct CudaBackend
 	// gs/gs_renderer.cpp:2395-2415).
 	template <bool AA, bool MIP>
 	void launch_shade(const PassParams &P, const DevInstance &I, uint32_t ns_log2, uint32_t grid,
-	                  const uint32_t *masks, const uint32_t *summary)
+	                  const uint32_t *masks, const uint32_t *summary, const uint32_t *d_flags)
 	{
 		if (I.rate_y_log2 != 0)
 		{
@@ -1156,15 +1145,17 @@ struct CudaBackend
 		if (I.rate_y_log2 != 0 && 2u + (1u << ns_log2) > num_planes)
 			return PGS_ERROR_INVALID_ARGUMENT;
 		size_t mask_words = subs * I.mask_words, summary_words = subs * I.summary_words;
-		int r = ensure_masks(mask_words + summary_words, tiles);
+		// Sub-tile masks, their summaries and the coarse tiles' flags, cleared together.
+		int r = ensure_masks(mask_words + summary_words + tiles);
 		if (r)
 			return r;
-		uint32_t *d_sub_masks = d_masks, *d_sub_summary = d_masks + mask_words;
+		uint32_t *d_sub_masks = d_masks, *d_sub_summary = d_masks + mask_words, *d_flags = d_sub_summary + summary_words;
 		{
 			StageScope ts(this, PGS_TIMESTAMP_BINNING);
-			CUDA_TRY(cudaMemsetAsync(d_masks, 0, (mask_words + summary_words) * sizeof(uint32_t), stream));
-			CUDA_TRY(cudaMemsetAsync(d_flags, 0, tiles * sizeof(uint32_t), stream));
-			bin_kernel<<<(count + 31) / 32, 32 * BIN_GROUP_WARPS, 0, stream>>>(P, I, d_sub_masks, d_sub_summary, d_flags);
+			CUDA_TRY(cudaMemsetAsync(d_masks, 0, (mask_words + summary_words + tiles) * sizeof(uint32_t), stream));
+			// A pass of few primitives spreads each group's candidates over more CTAs.
+			const uint32_t groups = (count + 31) / 32, slices = std::min(std::max(BIN_TARGET_CTAS / groups, 1u), 16u);
+			bin_kernel<<<dim3(groups, slices), 32 * BIN_GROUP_WARPS, 0, stream>>>(P, I, d_sub_masks, d_sub_summary, d_flags);
 			launch_counter++;
 		}
 		uint32_t grid = uint32_t(subs);
@@ -1194,11 +1185,11 @@ struct CudaBackend
 		// variant too (three variants per rate).
 		StageScope ts(this, PGS_TIMESTAMP_SHADING);
 		if (p.has_mipmap || p.has_ss_textures)
-			launch_shade<true, true>(P, I, ns_log2, grid, d_sub_masks, d_sub_summary);
+			launch_shade<true, true>(P, I, ns_log2, grid, d_sub_masks, d_sub_summary, d_flags);
 		else if (p.has_aa1)
-			launch_shade<true, false>(P, I, ns_log2, grid, d_sub_masks, d_sub_summary);
+			launch_shade<true, false>(P, I, ns_log2, grid, d_sub_masks, d_sub_summary, d_flags);
 		else
-			launch_shade<false, false>(P, I, ns_log2, grid, d_sub_masks, d_sub_summary);
+			launch_shade<false, false>(P, I, ns_log2, grid, d_sub_masks, d_sub_summary, d_flags);
 		CUDA_TRY(cudaGetLastError());
 		if (shade_timing)
 			return record_timing_event(shade_ev[1]);

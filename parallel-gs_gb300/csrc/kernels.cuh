@@ -292,6 +292,20 @@ __device__ __forceinline__ bool order_less(int32_t ax, int32_t ay, int32_t bx, i
 	return ax < bx;
 }
 
+// Inclusive sum over the lanes of a warp.
+__device__ __forceinline__ uint32_t warp_scan(uint32_t v, uint32_t lane)
+{
+	uint32_t x = v;
+	#pragma unroll
+	for (int o = 1; o < 32; o <<= 1)
+	{
+		const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+		if (lane >= uint32_t(o))
+			x += y;
+	}
+	return x;
+}
+
 template <typename T>
 __device__ __forceinline__ void dswap(T &a, T &b) { T t = a; a = b; b = t; }
 
@@ -969,132 +983,146 @@ __device__ __forceinline__ bool intersects_tile(const PrimSetup &s, int32_t lo0,
 // membership test and super-sampling flags (binning.comp:74-125); shading
 // lists are kept per 8x8 sub-tile as bitmasks over the pass's primitive range
 // so that ascending primitive order needs no sort.  A summary bitmask marks
-// non-empty mask words.  A CTA takes 32 primitives (one mask word): each of
-// its BIN_GROUP_WARPS warps loads all 32, warp 0 marks the coarse tiles, and
-// the warps share the (primitive, sub-tile) tests, so that the dependent
-// loads and shuffles of one batch overlap those of the others.
+// non-empty mask words.  The primitives of one mask word (32) are a group; its
+// (primitive, tile) candidates, those of the coarse grid and then those of the
+// sub-tile grid, are dealt out 32 at a time to the warps of gridDim.y CTAs, so
+// that neither a primitive over the whole frame nor one over hundreds of coarse
+// tiles holds a lane.
+// Bound: latency (dependent loads, shuffles and reductions at under 20 % of the
+// issue slots), hence many short chains: with one lane walking all coarse tiles
+// of its primitive and one CTA per group, a 61-primitive frame with a clear of
+// the whole frame took 47 us here and takes 4; the feedback frame's passes at 8x went from 15 to 4.6
 constexpr uint32_t BIN_GROUP_WARPS = 4;
+// CTAs a launch aims at when its groups are fewer (four per SM), up to 16 per group.
+constexpr uint32_t BIN_TARGET_CTAS = 608;
+
+// One live primitive of a group, as the dealt-out tests read it.
+struct BinItem
+{
+	PrimSetup s;
+	uint32_t local;   // index in the dispatch's primitive range
+	uint32_t ms_tri;
+	uint32_t flags;   // what the primitive adds to a coarse tile's flags
+	int32_t x0, y0, x1, y1; // its box inside the instance, relative to the instance's origin
+};
+
+// The items' candidate tiles of 2^shift pixels, dealt to the lanes: body(item,
+// tile x, tile y) runs for every tile of every item's box.  All lanes of the
+// calling warp take part.
+template <typename F>
+__device__ __forceinline__ void deal_tiles(const BinItem *items, uint32_t n, int shift, F &&body)
+{
+	const unsigned full = 0xffffffffu;
+	const uint32_t lane = threadIdx.x & 31u;
+	int32_t gx0 = 0, gy0 = 0, gw = 0;
+	uint32_t count = 0;
+	if (lane < n)
+	{
+		const BinItem &it = items[lane];
+		gx0 = it.x0 >> shift;
+		gy0 = it.y0 >> shift;
+		gw = (it.x1 >> shift) - gx0 + 1;
+		count = uint32_t(gw) * uint32_t((it.y1 >> shift) - gy0 + 1);
+	}
+	const uint32_t incl = warp_scan(count, lane), start = incl - count;
+	const uint32_t total = __shfl_sync(full, incl, 31);
+	const float inv = 1.0f / float(gw > 0 ? gw : 1);
+	const uint32_t first = (blockIdx.y * BIN_GROUP_WARPS + (threadIdx.x >> 5)) * 32u;
+	for (uint32_t base = first; base < total; base += 32u * BIN_GROUP_WARPS * gridDim.y)
+	{
+		// Every item has a candidate, so the starts are distinct: the owner of a
+		// candidate is the last item that starts at or before it.
+		const uint32_t before = __popc(__ballot_sync(full, count && start < base));
+		const uint32_t here = __reduce_or_sync(full, count && start - base < 32u ? 1u << (start - base) : 0u);
+		const uint32_t o = before + __popc(here & (2u << lane) - 1u) - 1u;
+		const uint32_t k = base + lane - __shfl_sync(full, start, int(o & 31u));
+		const int32_t o_gw = __shfl_sync(full, gw, int(o & 31u));
+		const float o_inv = __shfl_sync(full, inv, int(o & 31u));
+		const int32_t o_gx0 = __shfl_sync(full, gx0, int(o & 31u)), o_gy0 = __shfl_sync(full, gy0, int(o & 31u));
+		if (base + lane >= total)
+			continue;
+		// k / gw for k below 2^17 and gw up to 512: half a unit away from the
+		// next integer at k + 0.5, far more than the product's rounding.
+		const int32_t row = int32_t((float(k) + 0.5f) * o_inv);
+		body(items[o], o_gx0 + int32_t(k) - row * o_gw, o_gy0 + row);
+	}
+}
 
 __global__ void __launch_bounds__(32 * BIN_GROUP_WARPS) bin_kernel(PassParams P, DevInstance I, uint32_t *sub_masks,
                                                                    uint32_t *sub_summary, uint32_t *tile_flags)
 {
-	const unsigned full = 0xffffffffu;
-	const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-	const uint32_t local = blockIdx.x * 32u + lane;
-	const uint32_t p = I.prim_lo + local;
-	bool live = local < I.prim_count;
-	pgs_primitive_attribute pa = {};
-	PrimSetup s = {};
-	if (live)
-	{
-		pa = P.prims[p];
-		live = ((pa.state >> STATE_VERTEX_RENDER_PASS_INSTANCE_OFFSET) & 7u) == I.instance;
-	}
-	if (live)
-	{
-		s = P.setup[p];
-		live = !(s.bb[2] < s.bb[0] || s.bb[3] < s.bb[1]);
-	}
-
+	__shared__ BinItem items[32];
+	__shared__ uint32_t s_n;
+	const uint32_t lane = threadIdx.x & 31u;
 	const int ts = int(P.tile_size_log2);
-	const bool ms_tri = ((pa.state >> STATE_BIT_MULTISAMPLE) & 1) && !((pa.state >> STATE_BIT_LINE) & 1);
-	// Coarse tiles: membership and super-sampling flags, one primitive per
-	// thread of warp 0.
-	if (warp == 0 && live)
+	if (threadIdx.x < 32u)
 	{
-		int32_t tx0 = max((s.bb[0] - I.base_x) >> ts, 0), ty0 = max((s.bb[1] - I.base_y) >> ts, 0);
-		int32_t tx1 = min((s.bb[2] - I.base_x) >> ts, int32_t(I.tiles_w) - 1);
-		int32_t ty1 = min((s.bb[3] - I.base_y) >> ts, int32_t(I.tiles_h) - 1);
-		uint32_t flags = TILE_NONEMPTY;
-		if (I.rate_y_log2 != 0)
+		const uint32_t local = blockIdx.x * 32u + lane, p = I.prim_lo + local;
+		BinItem it;
+		bool live = false;
+		if (local < I.prim_count)
 		{
-			const uint32_t full_mask = (1u << STATE_BIT_SNAP_RASTER) | (1u << STATE_BIT_Z_TEST) | (1u << STATE_BIT_OPAQUE);
-			const uint32_t color_mask = (1u << STATE_BIT_SNAP_RASTER) | (1u << STATE_BIT_OPAQUE);
-			if ((pa.state & full_mask) != color_mask) flags |= TILE_REQ_SS_ZW;
-			if ((pa.state & color_mask) != color_mask) flags |= TILE_REQ_SS;
-			if (pa.state & (1u << STATE_BIT_Z_WRITE)) flags |= TILE_HAS_ZW;
-			if (pa.tex & TEX_PER_SAMPLE_BIT) flags |= TILE_REQ_SS;
-		}
-		for (int32_t ty = ty0; ty <= ty1; ty++)
-			for (int32_t tx = tx0; tx <= tx1; tx++)
+			const pgs_primitive_attribute pa = P.prims[p];
+			it.s = P.setup[p];
+			it.local = local;
+			it.ms_tri = ((pa.state >> STATE_BIT_MULTISAMPLE) & 1) && !((pa.state >> STATE_BIT_LINE) & 1);
+			it.flags = TILE_NONEMPTY;
+			if (I.rate_y_log2 != 0)
 			{
-				int32_t lo0 = I.base_x + (tx << ts), lo1 = I.base_y + (ty << ts);
-				if (!intersects_tile(s, lo0, lo1, lo0 + (1 << ts) - 1, lo1 + (1 << ts) - 1, ms_tri))
-					continue;
-				uint32_t tile = uint32_t(ty) * I.tiles_w + uint32_t(tx);
-				atomicOr(&tile_flags[tile], flags);
-				if (I.blend_demote)
-					atomicAdd(&tile_flags[tile], 1u << TILE_COUNT_SHIFT);
+				const uint32_t full_mask = (1u << STATE_BIT_SNAP_RASTER) | (1u << STATE_BIT_Z_TEST) | (1u << STATE_BIT_OPAQUE);
+				const uint32_t color_mask = (1u << STATE_BIT_SNAP_RASTER) | (1u << STATE_BIT_OPAQUE);
+				if ((pa.state & full_mask) != color_mask) it.flags |= TILE_REQ_SS_ZW;
+				if ((pa.state & color_mask) != color_mask) it.flags |= TILE_REQ_SS;
+				if (pa.state & (1u << STATE_BIT_Z_WRITE)) it.flags |= TILE_HAS_ZW;
+				if (pa.tex & TEX_PER_SAMPLE_BIT) it.flags |= TILE_REQ_SS;
 			}
+			it.x0 = max(it.s.bb[0] - I.base_x, 0);
+			it.y0 = max(it.s.bb[1] - I.base_y, 0);
+			it.x1 = min(it.s.bb[2] - I.base_x, int32_t(I.tiles_w << ts) - 1);
+			it.y1 = min(it.s.bb[3] - I.base_y, int32_t(I.tiles_h << ts) - 1);
+			live = ((pa.state >> STATE_VERTEX_RENDER_PASS_INSTANCE_OFFSET) & 7u) == I.instance && it.s.bb[2] >= it.s.bb[0] &&
+			       it.s.bb[3] >= it.s.bb[1] && it.x1 >= it.x0 && it.y1 >= it.y0;
+		}
+		const uint32_t alive = __ballot_sync(0xffffffffu, live);
+		if (live)
+			items[__popc(alive & ((1u << lane) - 1u))] = it;
+		if (lane == 0)
+			s_n = uint32_t(__popc(alive));
 	}
+	__syncthreads();
+	const uint32_t n = s_n;
+	if (!n)
+		return;
 
-	// 8x8 sub-tiles: the warp's (primitive, sub-tile) candidates are dealt out
-	// to its lanes 32 at a time, so one large primitive does not hold the warp.
+	auto mark_tile = [&](const BinItem &it, uint32_t tile) {
+		atomicOr(&tile_flags[tile], it.flags);
+		if (I.blend_demote)
+			atomicAdd(&tile_flags[tile], 1u << TILE_COUNT_SHIFT);
+	};
+	if (ts > 3)
+		deal_tiles(items, n, ts, [&](const BinItem &it, int32_t tx, int32_t ty) {
+			const int32_t lo0 = I.base_x + (tx << ts), lo1 = I.base_y + (ty << ts);
+			if (intersects_tile(it.s, lo0, lo1, lo0 + (1 << ts) - 1, lo1 + (1 << ts) - 1, it.ms_tri))
+				mark_tile(it, uint32_t(ty) * I.tiles_w + uint32_t(tx));
+		});
+
 	// A sub-tile that passes the test lies in a coarse tile that passes it
 	// (the test is monotonic in the rectangle), so testing the sub-tiles of the
 	// primitive's box inside the instance is the same as testing those of its
-	// member coarse tiles.
-	int32_t gx0 = 0, gy0 = 0, gw = 0, gh = 0;
-	if (live)
-	{
-		const int32_t xmax = I.base_x + int32_t(I.tiles_w << ts) - 1, ymax = I.base_y + int32_t(I.tiles_h << ts) - 1;
-		const int32_t x0 = max(s.bb[0], I.base_x), y0 = max(s.bb[1], I.base_y);
-		const int32_t x1 = min(s.bb[2], xmax), y1 = min(s.bb[3], ymax);
-		if (x1 >= x0 && y1 >= y0)
-		{
-			gx0 = (x0 - I.base_x) >> 3;
-			gy0 = (y0 - I.base_y) >> 3;
-			gw = ((x1 - I.base_x) >> 3) - gx0 + 1;
-			gh = ((y1 - I.base_y) >> 3) - gy0 + 1;
-		}
-	}
-	const uint32_t count = uint32_t(gw * gh);
-	uint32_t incl = count;
-	#pragma unroll
-	for (int o = 1; o < 32; o <<= 1)
-	{
-		const uint32_t y = __shfl_up_sync(full, incl, o);
-		if (lane >= uint32_t(o))
-			incl += y;
-	}
-	const uint32_t total = __shfl_sync(full, incl, 31);
-	const uint32_t warp_first = blockIdx.x * 32u;
-	for (uint32_t base = warp * 32u; base < total; base += 32u * BIN_GROUP_WARPS)
-	{
-		const uint32_t j = base + lane;
-		// Owner: the first lane whose inclusive count exceeds j.
-		uint32_t lo = 0, hi = 31;
-		#pragma unroll
-		for (int it = 0; it < 5; it++)
-		{
-			const uint32_t mid = (lo + hi) >> 1;
-			const uint32_t v = __shfl_sync(full, incl, int(mid));
-			if (v > j)
-				hi = mid;
-			else
-				lo = mid + 1u;
-		}
-		const uint32_t o = lo;
-		const uint32_t o_incl = __shfl_sync(full, incl, int(o)), o_count = __shfl_sync(full, count, int(o));
-		const int32_t o_gx0 = __shfl_sync(full, gx0, int(o)), o_gy0 = __shfl_sync(full, gy0, int(o));
-		const int32_t o_gw = __shfl_sync(full, gw, int(o));
-		const bool o_ms = __shfl_sync(full, ms_tri ? 1 : 0, int(o)) != 0;
-		if (j >= total)
-			continue;
-		const uint32_t k = j - (o_incl - o_count);
-		const int32_t gx = o_gx0 + int32_t(k % uint32_t(o_gw)), gy = o_gy0 + int32_t(k / uint32_t(o_gw));
-		const uint32_t o_local = warp_first + o;
-		const PrimSetup &os = P.setup[I.prim_lo + o_local];
+	// member coarse tiles.  Coarse tiles of 8x8 pixels are the sub-tiles.
+	deal_tiles(items, n, 3, [&](const BinItem &it, int32_t gx, int32_t gy) {
 		const int32_t sx = I.base_x + (gx << 3), sy = I.base_y + (gy << 3);
-		if (!intersects_tile(os, sx, sy, sx + 7, sy + 7, o_ms))
-			continue;
+		if (!intersects_tile(it.s, sx, sy, sx + 7, sy + 7, it.ms_tri))
+			return;
 		// Results unused: both compile to fire-and-forget reductions.
-		const uint32_t word = o_local >> 5, bit = 1u << (o_local & 31u);
+		const uint32_t word = it.local >> 5, bit = 1u << (it.local & 31u);
 		const uint32_t sword = word >> 5, sbit = 1u << (word & 31u);
 		const size_t sub = size_t(gy) * I.sub_w + size_t(gx);
 		atomicOr(&sub_masks[sub * I.mask_words + word], bit);
 		atomicOr(&sub_summary[sub * I.summary_words + sword], sbit);
-	}
+		if (ts == 3)
+			mark_tile(it, uint32_t(sub));
+	});
 }
 
 // ---------------------------------------------------------------------------
@@ -2592,19 +2620,6 @@ struct ListScan
 {
 	uint32_t lo, hi, total;
 };
-
-__device__ __forceinline__ uint32_t warp_scan(uint32_t v, uint32_t lane)
-{
-	uint32_t x = v;
-	#pragma unroll
-	for (int o = 1; o < 32; o <<= 1)
-	{
-		const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-		if (lane >= uint32_t(o))
-			x += y;
-	}
-	return x;
-}
 
 template <uint32_t WARPS>
 __device__ __forceinline__ ListScan list_scan(const DevInstance &I, const uint32_t *summary, const uint32_t *mask, ListShared &L)
