@@ -414,7 +414,7 @@ class GSInterface:
         """RGBA8 image (height, width, 4) of CRTC circuit 0 or 1."""
         w, h = C.c_uint32(), C.c_uint32()
         cap = 4096 * 4096 * 4
-        out = np.zeros(cap, dtype=np.uint8)
+        out = np.empty(cap, dtype=np.uint8)  # only the circuit's rectangle is used
         check(self.lib.pgs_gs_scanout_circuit(self.handle, circuit, phase, flags, out.ctypes.data, cap, C.byref(w),
                                               C.byref(h)), "scanout_circuit")
         return out[: w.value * h.value * 4].reshape(h.value, w.value, 4).copy()
@@ -427,7 +427,9 @@ class GSInterface:
         info = VsyncInfo(phase, flags)
         res = ScanoutResult()
         cap = 3840 * 2160 * 4
-        out = np.zeros(cap, dtype=np.uint8)
+        # Not zeroed: clearing 33 MB costs many times what the read-out does, and
+        # only the result's width x height x 4 bytes are used.
+        out = np.empty(cap, dtype=np.uint8)
         check(self.lib.pgs_gs_vsync(self.handle, C.byref(info), out.ctypes.data, cap, C.byref(res)), "vsync")
         d = {k: getattr(res, k) for k, _ in ScanoutResult._fields_ if k != "padding"}
         img = out[: res.width * res.height * 4].reshape(res.height, res.width, 4).copy()
