@@ -39,6 +39,8 @@ constexpr int REAL_IN[LAYERS] = { 4, 32, 32, 32, 32, 32 };
 constexpr int REAL_OUT[LAYERS] = { 32, 32, 32, 32, 32, 4 };
 constexpr int PAD_IN[LAYERS] = { 16, 32, 32, 32, 32, 32 };
 constexpr int PAD_OUT[LAYERS] = { 32, 32, 32, 32, 32, 8 };
+// Floats per layer of the padded weight and bias gradients.
+constexpr size_t WGRAD_STRIDE = 9 * 32 * 32, BGRAD_STRIDE = 32;
 // Device copies of the layer shapes.
 __constant__ int d_real_in[LAYERS] = { 4, 32, 32, 32, 32, 32 };
 __constant__ int d_real_out[LAYERS] = { 32, 32, 32, 32, 32, 4 };
@@ -299,8 +301,17 @@ __global__ void __launch_bounds__(256) conv3x3_kernel(ConvArgs A)
 
 // Weight gradient dW[tap][co][ci] += sum_p X[p + off(tap)][ci] * dY[p][co]
 // (stored in the forward layout).  Each CTA walks 16x16 pixel tiles with a
-// grid stride and accumulates all nine taps in shared memory before one
-// global atomic per element.
+// grid stride; one warp per tap keeps its tap's COUT x CIN sums in registers
+// for the whole launch and adds them to global memory once.  A tile's halo of X
+// and its dY are copied asynchronously into one of two buffers while the other
+// is multiplied.  A tile's 16 k16 steps are summed by the tensor cores, the
+// tiles' sums in FP32.
+// Bound: shared-memory reads of the fragments (about 2300 cycles a tile) next to
+// the legacy MMA's rate.  The version with a shared-memory sum that every warp
+// added each tap of each tile to, and one thread per channel for the bias, took
+// 138 us for a 32 -> 32 layer of 16 128x128 crops; this takes 23 us.  The bias
+// goes to global memory once per CTA: once per warp and channel, on one cache
+// line, took 64 us.  One CTA per SM: 27 us.
 struct WgradArgs
 {
 	const __nv_bfloat16 *x;   // N x H x W x CIN (layer input)
@@ -310,130 +321,164 @@ struct WgradArgs
 	int n, h, w;
 };
 
+constexpr int WGRAD_THREADS = 9 * 32;
+constexpr int WGRAD_CTAS = 2; // per SM
+
+// One buffer: the halo of X, then the tile of dY, rows padded by 16 bytes.
 template <int CIN, int COUT>
-constexpr size_t wgrad_smem_bytes()
+__host__ __device__ constexpr size_t wgrad_buffer_bytes()
 {
-	return (9 * COUT * CIN + 32) * 4 + (HALO * HALO * (CIN + 8) + TILE * TILE * (COUT + 8)) * 2;
+	return (HALO * HALO * (CIN + 8) + TILE * TILE * (COUT + 8)) * 2;
+}
+
+// 16 bytes from global to shared memory, or zeros.
+__device__ __forceinline__ void cp_async16(void *dst, const void *src, bool valid)
+{
+	asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(smem_u32(dst)), "l"(src), "r"(valid ? 16 : 0) : "memory");
 }
 
 template <int CIN, int COUT>
-__global__ void __launch_bounds__(256) wgrad_kernel(WgradArgs A)
+__global__ void __launch_bounds__(WGRAD_THREADS, 2) wgrad_kernel(WgradArgs A)
 {
 	constexpr int PS = CIN + 8;
 	constexpr int PD = COUT + 8;
-	constexpr int MT = CIN / 16;    // m16 tiles over input channels
-	constexpr int NT = COUT / 8;    // n8 tiles over output channels
-	// Dynamic shared memory (over the 48 KiB static limit): the nine-tap
-	// accumulator, the halo of X and the tile of dY.
+	constexpr int MT = COUT / 16;   // m16 tiles over output channels
+	constexpr int NT = CIN / 8;     // n8 tiles over input channels
+	constexpr int CHUNKS = COUT / 8;
 	extern __shared__ __align__(16) uint8_t smem_raw[];
-	float *s_dw = reinterpret_cast<float *>(smem_raw);
-	float *s_db = s_dw + 9 * COUT * CIN;
-	__nv_bfloat16 *s_x = reinterpret_cast<__nv_bfloat16 *>(s_db + 32);
-	__nv_bfloat16 *s_dy = s_x + HALO * HALO * PS;
 
 	const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-	for (int i = tid; i < 9 * COUT * CIN; i += 256)
-		s_dw[i] = 0.0f;
-	if (tid < COUT)
-		s_db[tid] = 0.0f;
-
 	const int tiles_x = (A.w + TILE - 1) / TILE, tiles_y = (A.h + TILE - 1) / TILE;
 	const int tiles = tiles_x * tiles_y * A.n;
-	for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x)
-	{
+	auto buffer_x = [&](int b) { return reinterpret_cast<__nv_bfloat16 *>(smem_raw + b * wgrad_buffer_bytes<CIN, COUT>()); };
+	auto load = [&](int tile, int b) {
 		const int img = tile / (tiles_x * tiles_y), rem = tile % (tiles_x * tiles_y);
 		const int x0 = (rem % tiles_x) * TILE, y0 = (rem / tiles_x) * TILE;
-		__syncthreads();
-		for (int i = tid; i < HALO * HALO * (CIN / 8); i += 256)
+		__nv_bfloat16 *s_x = buffer_x(b), *s_dy = s_x + HALO * HALO * PS;
+		for (int i = tid; i < HALO * HALO * (CIN / 8); i += WGRAD_THREADS)
 		{
-			int p = i / (CIN / 8), c = (i % (CIN / 8)) * 8;
-			int gx = x0 - 1 + p % HALO, gy = y0 - 1 + p / HALO;
-			uint4 v = make_uint4(0, 0, 0, 0);
-			if (gx >= 0 && gy >= 0 && gx < A.w && gy < A.h)
-				v = *reinterpret_cast<const uint4 *>(A.x + ((size_t(img) * A.h + gy) * A.w + gx) * CIN + c);
-			*reinterpret_cast<uint4 *>(s_x + p * PS + c) = v;
+			const int p = i / (CIN / 8), c = (i % (CIN / 8)) * 8;
+			const int gx = x0 - 1 + p % HALO, gy = y0 - 1 + p / HALO;
+			const bool in = gx >= 0 && gy >= 0 && gx < A.w && gy < A.h;
+			cp_async16(s_x + p * PS + c, in ? A.x + ((size_t(img) * A.h + gy) * A.w + gx) * CIN + c : A.x, in);
 		}
-		for (int i = tid; i < TILE * TILE * (COUT / 8); i += 256)
+		for (int i = tid; i < TILE * TILE * CHUNKS; i += WGRAD_THREADS)
 		{
-			int p = i / (COUT / 8), c = (i % (COUT / 8)) * 8;
-			int gx = x0 + p % TILE, gy = y0 + p / TILE;
-			uint4 v = make_uint4(0, 0, 0, 0);
-			if (gx < A.w && gy < A.h)
-				v = *reinterpret_cast<const uint4 *>(A.dy + ((size_t(img) * A.h + gy) * A.w + gx) * COUT + c);
-			*reinterpret_cast<uint4 *>(s_dy + p * PD + c) = v;
+			const int p = i / CHUNKS, c = (i % CHUNKS) * 8;
+			const int gx = x0 + p % TILE, gy = y0 + p / TILE;
+			const bool in = gx < A.w && gy < A.h;
+			cp_async16(s_dy + p * PD + c, in ? A.dy + ((size_t(img) * A.h + gy) * A.w + gx) * COUT + c : A.dy, in);
 		}
-		__syncthreads();
+		asm volatile("cp.async.commit_group;\n" ::: "memory");
+	};
 
-		// Bias gradient: column sums of dY (pixels outside the image are zero).
-		if (tid < COUT)
+	float sum[MT][NT][4] = {};
+	// Bias gradient: column sums of dY (pixels outside the image are zero), 8
+	// channels of every 256 / CHUNKS-th pixel per thread.
+	float bias[8] = {};
+	const int dy = warp / 3, dx = warp % 3;
+	if (int(blockIdx.x) < tiles)
+		load(blockIdx.x, 0);
+	for (int tile = blockIdx.x, b = 0; tile < tiles; tile += gridDim.x, b ^= 1)
+	{
+		asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+		// This tile has arrived for all, and all are done with the other buffer.
+		__syncthreads();
+		if (tile + int(gridDim.x) < tiles)
+			load(tile + gridDim.x, b ^ 1);
+		const __nv_bfloat16 *s_x = buffer_x(b), *s_dy = s_x + HALO * HALO * PS;
+		if (tid < 256)
 		{
-			float s = 0.0f;
-			for (int p = 0; p < TILE * TILE; p++)
-				s += __bfloat162float(s_dy[p * PD + tid]);
-			s_db[tid] += s;
+			const int c = tid % CHUNKS;
+			#pragma unroll
+			for (int p = tid / CHUNKS; p < TILE * TILE; p += 256 / CHUNKS)
+			{
+				const uint4 v = *reinterpret_cast<const uint4 *>(s_dy + p * PD + c * 8);
+				const uint32_t q[4] = { v.x, v.y, v.z, v.w };
+				#pragma unroll
+				for (int k = 0; k < 4; k++)
+				{
+					bias[2 * k] += __uint_as_float(q[k] << 16);
+					bias[2 * k + 1] += __uint_as_float(q[k] & 0xffff0000u);
+				}
+			}
 		}
-
-		// Warp: pixel rows 2w, 2w+1 (K = 32 pixels, two k16 steps).
-		#pragma unroll 1
-		for (int tap = 0; tap < 9; tap++)
+		float acc[MT][NT][4] = {};
+		#pragma unroll 4
+		for (int row = 0; row < TILE; row++)
 		{
-			const int dy = tap / 3, dx = tap % 3;
-			float acc[MT][NT][4];
+			// The 16 pixels of one tile row are one k16 step.
+			// A (m = output channel, k = pixel): transposed 8x8 loads from
+			// pixel-major memory.  Matrix q: pixels (q >> 1) * 8 + 0..7,
+			// channels (q & 1) * 8 + 0..7.
+			const int q = lane >> 3;
+			uint32_t a[MT][4];
 			#pragma unroll
 			for (int m = 0; m < MT; m++)
-				#pragma unroll
-				for (int j = 0; j < NT; j++)
-					#pragma unroll
-					for (int k = 0; k < 4; k++)
-						acc[m][j][k] = 0.0f;
+				ldsm_x4_t(smem_u32(s_dy + (row * TILE + (q >> 1) * 8 + (lane & 7)) * PD + m * 16 + (q & 1) * 8), a[m][0], a[m][1],
+				          a[m][2], a[m][3]);
+			// B (k = pixel, n = input channel), two n8 tiles per load: matrix q
+			// has pixels (q & 1) * 8 + 0..7 of channels (q >> 1) * 8 + 0..7.
 			#pragma unroll
-			for (int ks = 0; ks < 2; ks++)
+			for (int j = 0; j < NT; j += 2)
 			{
-				const int row = warp * 2 + ks;   // the 16 pixels of one tile row are one k16 step
-				// A (m = input channel, k = pixel): transposed 8x8 loads from
-				// pixel-major memory.  Matrix q: pixels (q >> 1) * 8 + 0..7,
-				// channels (q & 1) * 8 + 0..7.
-				uint32_t a[MT][4];
+				uint32_t b0, b1, b2, b3;
+				ldsm_x4_t(smem_u32(s_x + ((row + dy) * HALO + dx + (q & 1) * 8 + (lane & 7)) * PS + (j + (q >> 1)) * 8), b0, b1, b2,
+				          b3);
 				#pragma unroll
 				for (int m = 0; m < MT; m++)
 				{
-					int q = lane >> 3, px = (q >> 1) * 8 + (lane & 7);
-					const __nv_bfloat16 *p = s_x + ((row + dy) * HALO + px + dx) * PS + m * 16 + (q & 1) * 8;
-					ldsm_x4_t(smem_u32(p), a[m][0], a[m][1], a[m][2], a[m][3]);
-				}
-				// B (k = pixel, n = output channel): transposed loads from
-				// pixel-major dY; lanes 0-7 pixels 0-7, lanes 8-15 pixels 8-15.
-				#pragma unroll
-				for (int j = 0; j < NT; j++)
-				{
-					int px = ((lane >> 3) & 1) * 8 + (lane & 7);
-					const __nv_bfloat16 *p = s_dy + (row * TILE + px) * PD + j * 8;
-					uint32_t b0, b1;
-					ldsm_x2_t(smem_u32(p), b0, b1);
-					#pragma unroll
-					for (int m = 0; m < MT; m++)
-						mma_bf16(acc[m][j], a[m], b0, b1);
+					mma_bf16(acc[m][j], a[m], b0, b1);
+					mma_bf16(acc[m][j + 1], a[m], b2, b3);
 				}
 			}
-			// acc[m][j]: rows (ci) m*16 + g (+8), columns (co) j*8 + 2t (+1).
-			const int g = lane >> 2, t = lane & 3;
+		}
+		#pragma unroll
+		for (int m = 0; m < MT; m++)
 			#pragma unroll
-			for (int m = 0; m < MT; m++)
+			for (int j = 0; j < NT; j++)
 				#pragma unroll
-				for (int j = 0; j < NT; j++)
-					#pragma unroll
-					for (int k = 0; k < 4; k++)
-					{
-						int ci = m * 16 + g + (k >> 1) * 8, co = j * 8 + 2 * t + (k & 1);
-						atomicAdd(&s_dw[(tap * COUT + co) * CIN + ci], acc[m][j][k]);
-					}
+				for (int k = 0; k < 4; k++)
+					sum[m][j][k] += acc[m][j][k];
+	}
+	// sum[m][j]: rows (co) m*16 + g (+8), columns (ci) j*8 + 2t (+1).
+	const int g = lane >> 2, t = lane & 3;
+	#pragma unroll
+	for (int m = 0; m < MT; m++)
+		#pragma unroll
+		for (int j = 0; j < NT; j++)
+			#pragma unroll
+			for (int half = 0; half < 2; half++)
+			{
+				float *dst = A.dw + (warp * COUT + m * 16 + g + half * 8) * CIN + j * 8 + 2 * t;
+				asm volatile("red.global.add.v2.f32 [%0], {%1, %2};\n" ::"l"(dst), "f"(sum[m][j][2 * half]),
+				             "f"(sum[m][j][2 * half + 1])
+				             : "memory");
+			}
+	// Bias: lanes of a warp with the same chunk, then the warps, then one
+	// addition per CTA and channel (all of them fall on one cache line).
+	__shared__ float s_db[8][COUT];
+	if (tid < 256)
+	{
+		#pragma unroll
+		for (int k = 0; k < 8; k++)
+		{
+			#pragma unroll
+			for (int o = CHUNKS; o < 32; o <<= 1)
+				bias[k] += __shfl_xor_sync(0xffffffffu, bias[k], o);
+			if (lane < CHUNKS)
+				s_db[warp][lane * 8 + k] = bias[k];
 		}
 	}
 	__syncthreads();
-	for (int i = tid; i < 9 * COUT * CIN; i += 256)
-		atomicAdd(&A.dw[i], s_dw[i]);
 	if (tid < COUT)
-		atomicAdd(&A.db[tid], s_db[tid]);
+	{
+		float v = 0.0f;
+		#pragma unroll
+		for (int k = 0; k < 8; k++)
+			v += s_db[k][tid];
+		atomicAdd(&A.db[tid], v);
+	}
 }
 
 // RGBA8 image -> BF16 16-channel input (channels 4..15 zero).
@@ -455,30 +500,38 @@ __global__ void __launch_bounds__(256) image_to_bf16_kernel(const uint8_t *img, 
 // MSE loss over the four channels against the target image, and its
 // gradient 2 (out - target) / count as BF16 16-channel input of the last
 // layer's backward pass.
+// One addition to the sum per CTA: a CTA per 256 pixels with one per warp spent
+// its time queueing 8192 additions at one address (16 crops of 128x128: 16.5 us
+// against 9.5).
 __global__ void __launch_bounds__(256) loss_kernel(const float *out, const uint8_t *target, size_t pixels, float scale,
                                                    __nv_bfloat16 *grad, double *loss_sum)
 {
-	size_t p = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
+	__shared__ double s_part[8];
 	double local = 0.0;
-	if (p < pixels)
+	for (size_t p = size_t(blockIdx.x) * 256 + threadIdx.x; p < pixels; p += size_t(gridDim.x) * 256)
 	{
-		uint32_t w[8] = {};
-		float d[4];
+		const float4 v = reinterpret_cast<const float4 *>(out)[p];
+		const uint32_t c = reinterpret_cast<const uint32_t *>(target)[p];
+		const float d[4] = { v.x - float(c & 0xffu) / 255.0f, v.y - float((c >> 8) & 0xffu) / 255.0f,
+		                     v.z - float((c >> 16) & 0xffu) / 255.0f, v.w - float(c >> 24) / 255.0f };
+		#pragma unroll
 		for (int k = 0; k < 4; k++)
-		{
-			d[k] = out[p * 4 + k] - float(target[p * 4 + k]) / 255.0f;
 			local += double(d[k]) * d[k];
-		}
-		w[0] = pack_bf16x2(scale * d[0], scale * d[1]);
-		w[1] = pack_bf16x2(scale * d[2], scale * d[3]);
 		uint4 *o = reinterpret_cast<uint4 *>(grad + p * 16);
-		o[0] = make_uint4(w[0], w[1], w[2], w[3]);
-		o[1] = make_uint4(w[4], w[5], w[6], w[7]);
+		o[0] = make_uint4(pack_bf16x2(scale * d[0], scale * d[1]), pack_bf16x2(scale * d[2], scale * d[3]), 0, 0);
+		o[1] = make_uint4(0, 0, 0, 0);
 	}
 	for (int o = 16; o > 0; o >>= 1)
 		local += __shfl_xor_sync(0xffffffffu, local, o);
 	if ((threadIdx.x & 31) == 0)
+		s_part[threadIdx.x >> 5] = local;
+	__syncthreads();
+	if (threadIdx.x == 0)
+	{
+		for (int k = 1; k < 8; k++)
+			local += s_part[k];
 		atomicAdd(loss_sum, local);
+	}
 }
 
 // Parameter block of one layer inside the flat FP32 parameter vector:
@@ -546,12 +599,15 @@ __global__ void __launch_bounds__(256) pack_weights_kernel(const float *params, 
 	}
 }
 
-// Gradient of the last layer from a [9][8][32] (padded) wgrad buffer is
-// produced directly in real layout by copying: wgrad kernels write padded
-// blocks that gather_grad_kernel folds into the flat gradient vector.
-__global__ void __launch_bounds__(256) gather_grad_kernel(const float *padded_w, const float *padded_b, int layer,
-                                                          int cout_pad, int cin_pad, float *grad)
+// The wgrad kernels write padded blocks of 32x32x9 weights and 32 biases per
+// layer; this folds them into the flat gradient vector (grid y = layer).
+__global__ void __launch_bounds__(256) gather_grad_kernel(const float *padded_w, const float *padded_b, float *grad)
 {
+	const int layer = blockIdx.y;
+	padded_w += layer * WGRAD_STRIDE;
+	padded_b += layer * BGRAD_STRIDE;
+	// Gradients at the last layer's output are padded to 16 channels.
+	const int cout_pad = layer == LAYERS - 1 ? 16 : 32, cin_pad = d_pad_in[layer];
 	int i = blockIdx.x * blockDim.x + threadIdx.x;
 	int real_out = d_real_out[layer], real_in = d_real_in[layer];
 	int nw = 9 * real_out * real_in;
@@ -923,7 +979,6 @@ struct Upscaler
 	LayerOffsets off = {};
 	float *d_params = nullptr, *d_m = nullptr, *d_v = nullptr, *d_grad = nullptr;
 	float *d_wgrad = nullptr, *d_bgrad = nullptr;   // padded scratch, per layer
-	size_t wgrad_stride = 9 * 32 * 32, bgrad_stride = 32;
 	BfLayout bf = {};
 	int adam_t = 0;
 	// Activations for the current batch size.
@@ -994,8 +1049,8 @@ struct Upscaler
 		UP_TRY(cudaMemset(d_params, 0, n * 4));
 		UP_TRY(cudaMemset(d_m, 0, n * 4));
 		UP_TRY(cudaMemset(d_v, 0, n * 4));
-		UP_TRY(cudaMalloc(&d_wgrad, LAYERS * wgrad_stride * 4));
-		UP_TRY(cudaMalloc(&d_bgrad, LAYERS * bgrad_stride * 4));
+		UP_TRY(cudaMalloc(&d_wgrad, LAYERS * WGRAD_STRIDE * 4));
+		UP_TRY(cudaMalloc(&d_bgrad, LAYERS * BGRAD_STRIDE * 4));
 		for (int l = 0; l < LAYERS; l++)
 		{
 			UP_TRY(cudaMalloc(&bf.fwd[l], size_t(9) * PAD_OUT[l] * PAD_IN[l] * 2));
@@ -1213,12 +1268,12 @@ struct Upscaler
 	template <int CIN, int COUT>
 	int wgrad(const __nv_bfloat16 *x, const __nv_bfloat16 *dy, int layer, int n, int h, int w)
 	{
-		WgradArgs a = { x, dy, d_wgrad + layer * wgrad_stride, d_bgrad + layer * bgrad_stride, n, h, w };
+		WgradArgs a = { x, dy, d_wgrad + layer * WGRAD_STRIDE, d_bgrad + layer * BGRAD_STRIDE, n, h, w };
 		int tiles = ((w + TILE - 1) / TILE) * ((h + TILE - 1) / TILE) * n;
-		int grid = std::min(tiles, sm_count * 2);
-		constexpr size_t smem = wgrad_smem_bytes<CIN, COUT>();
+		int grid = std::min(tiles, sm_count * WGRAD_CTAS);
+		constexpr size_t smem = 2 * wgrad_buffer_bytes<CIN, COUT>();
 		UP_TRY(cudaFuncSetAttribute(wgrad_kernel<CIN, COUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-		wgrad_kernel<CIN, COUT><<<grid, 256, smem, stream>>>(a);
+		wgrad_kernel<CIN, COUT><<<grid, WGRAD_THREADS, smem, stream>>>(a);
 		UP_TRY(cudaGetLastError());
 		return PGS_OK;
 	}
@@ -1232,10 +1287,10 @@ struct Upscaler
 			return r;
 		size_t pixels = size_t(n) * h * w;
 		UP_TRY(cudaMemsetAsync(d_loss, 0, sizeof(double), stream));
-		UP_TRY(cudaMemsetAsync(d_wgrad, 0, LAYERS * wgrad_stride * 4, stream));
-		UP_TRY(cudaMemsetAsync(d_bgrad, 0, LAYERS * bgrad_stride * 4, stream));
+		UP_TRY(cudaMemsetAsync(d_wgrad, 0, LAYERS * WGRAD_STRIDE * 4, stream));
+		UP_TRY(cudaMemsetAsync(d_bgrad, 0, LAYERS * BGRAD_STRIDE * 4, stream));
 		float scale = 2.0f / float(pixels * 4);
-		loss_kernel<<<unsigned((pixels + 255) / 256), 256, 0, stream>>>(d_out, d_target, pixels, scale, d_gout, d_loss);
+		loss_kernel<<<unsigned(std::min((pixels + 255) / 256, size_t(sm_count) * 4)), 256, 0, stream>>>(d_out, d_target, pixels, scale, d_gout, d_loss);
 		UP_TRY(cudaGetLastError());
 		// Layer 5: weight gradient from the 16-channel output gradient, data
 		// gradient into layer 4's output through its ReLU.
@@ -1266,15 +1321,8 @@ struct Upscaler
 		}
 		if ((r = wgrad<16, 32>(d_x0, g, 0, n, h, w)))
 			return r;
-		for (int l = 0; l < LAYERS; l++)
-		{
-			int cout_pad = l == LAYERS - 1 ? 16 : 32, cin_pad = PAD_IN[l];
-			int count = 9 * REAL_OUT[l] * REAL_IN[l] + REAL_OUT[l];
-			gather_grad_kernel<<<(count + 255) / 256, 256, 0, stream>>>(d_wgrad + l * wgrad_stride,
-			                                                            d_bgrad + l * bgrad_stride, l, cout_pad,
-			                                                            cin_pad, d_grad);
-			UP_TRY(cudaGetLastError());
-		}
+		gather_grad_kernel<<<dim3((9 * 32 * 32 + 32 + 255) / 256, LAYERS), 256, 0, stream>>>(d_wgrad, d_bgrad, d_grad);
+		UP_TRY(cudaGetLastError());
 		if (loss)
 		{
 			double s = 0.0;
