@@ -183,6 +183,27 @@ __device__ __forceinline__ void tma_load_4d(void *dst, const void *tmap, uint64_
 	             : "memory");
 }
 
+// 4-D TMA tile store from shared memory (elements outside the tensor are not
+// written), and the bulk groups that track such stores: commit what the thread
+// issued, wait until at most N groups still read their shared memory, wait until
+// all are complete.
+__device__ __forceinline__ void tma_store_4d(const void *tmap, const void *src, int32_t c0, int32_t c1, int32_t c2, int32_t c3)
+{
+	asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.bulk_group [%0, {%1, %2, %3, %4}], [%5];\n" ::"l"(tmap), "r"(c0),
+	             "r"(c1), "r"(c2), "r"(c3), "r"(smem_addr(src))
+	             : "memory");
+}
+
+__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;\n" ::: "memory"); }
+
+template <int N>
+__device__ __forceinline__ void bulk_wait_read()
+{
+	asm volatile("cp.async.bulk.wait_group.read %0;\n" ::"n"(N) : "memory");
+}
+
+__device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;\n" ::: "memory"); }
+
 // Byte offset of element (row, k) of a K-major BF16 tile stored with 64-byte
 // swizzle (rows of 32 elements).
 __host__ __device__ constexpr uint32_t swz64_offset(uint32_t row, uint32_t k)

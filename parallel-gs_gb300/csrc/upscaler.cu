@@ -711,54 +711,61 @@ __global__ void __launch_bounds__(128) umma_probe_kernel(uint32_t mode, float *o
 
 // ---------------------------------------------------------------------------
 // 32 -> 32 convolution on the 5th-generation tensor cores (inference and the
-// forward half of training).  Persistent CTAs (one per SM) own tiles of
-// 8 rows x 16 columns = 128 output pixels.  Warp-specialised pipeline:
-//  - warp 0, one lane: TMA loads of three copies of each tile's 10 x 16 x 32
-//    input window, shifted by dx = 0, 1, 2 columns (zero fill outside the
-//    image, 64-byte swizzle), so that for every tap the 128 A rows are
-//    contiguous; three input stages;
-//  - the same lane issues 9 taps x 2 K-steps of tcgen05.mma (M 128, N 32,
-//    K 16) into one of two 32-column FP32 accumulators in tensor memory and
-//    commits to the stage's "empty" and the accumulator's "full" barriers;
+// forward half of training).  Persistent CTAs own tiles of 16 rows x 8 columns
+// = 128 output pixels.  Warp-specialised pipeline:
+//  - warp 5, one lane: TMA loads of each tile's 18 x 10 x 32 input window (zero
+//    fill outside the image, 64-byte swizzle), five stages.  It is not the lane
+//    that issues the MMAs: refilling a stage waits for the MMAs that read it, and
+//    one lane for both let the tensor cores run dry at every tile;
+//  - warp 0, one lane: 9 taps x 2 K-steps of tcgen05.mma (M 128, N 32, K 16)
+//    into one of four 32-column FP32 accumulators in tensor memory, committed to
+//    the stage's "empty" and the accumulator's "full" barriers.  A
+//    row group of A is the 8 pixels of one window row from the tap's column on:
+//    groups lie one window row (640 bytes) apart, and since the swizzle is a
+//    function of the shared-memory address, a group may start at any pixel;
 //  - warps 1-4 (one per TMEM lane quarter) read the accumulator, release it,
-//    add the bias, apply ReLU and store BF16 NHWC rows, overlapping the MMAs
-//    of the next tile.
+//    add the bias, apply ReLU and hand their 8 x 4 pixels to a TMA store
+//    (clipped at the image border), overlapping the MMAs of the next tile.
 // The layer's weights sit in shared memory (9 x 32 x 32 BF16, 64-byte
 // swizzled) for the whole launch.  Every wait is bounded and gives up when
 // another warp has given up.
+// Bound: shared-memory reads of A, 4 KiB per MMA of 16 tensor cycles (a layer of
+// a 640x448 frame: 5.6 us), and the launch's start and end.  Measured on the
+// network of one such frame, 83 us at first: one window per tile instead of three
+// shifted by a column each (11.5 instead of 30 KB), boxes stored by TMA instead
+// of 16 bytes a lane, and unrolled descriptors, together 81.6; loads from a warp
+// of their own, 69.6.
 namespace tc
 {
-constexpr int ROWS = 8, COLS = 16, PIX = ROWS * COLS;
-constexpr int WIN_ROWS = ROWS + 2;
-constexpr int STAGES = 3, ACCS = 2;
-constexpr uint32_t COPY_BYTES = WIN_ROWS * COLS * 64;      // 10240
-constexpr uint32_t STAGE_BYTES = 3 * COPY_BYTES;            // 30720
+constexpr int ROWS = 16, COLS = 8;
+constexpr int WIN_ROWS = ROWS + 2, WIN_COLS = COLS + 2;
+constexpr int STAGES = 5, ACCS = 4;
+constexpr uint32_t ROW_BYTES = WIN_COLS * 64;               // 640
+constexpr uint32_t WIN_BYTES = WIN_ROWS * ROW_BYTES;        // 11520
+constexpr uint32_t STAGE_BYTES = 12288;                     // a window from a 1 KiB boundary
 constexpr uint32_t W_BYTES = 9 * 32 * 64;                   // 18432
-constexpr uint32_t SMEM_BYTES = 1024 + STAGES * STAGE_BYTES + W_BYTES + 1024;
-constexpr int THREADS = 160;
+constexpr uint32_t OUT_BYTES = 32 * 64;                     // one warp's 8 x 4 pixels
+constexpr int OUT_BUFS = 2;
+constexpr uint32_t SMEM_BYTES = 1024 + STAGES * STAGE_BYTES + W_BYTES + 4 * OUT_BUFS * OUT_BYTES;
+constexpr int THREADS = 192;
 }
 
-// Epilogue outputs of conv32_tc_kernel: EPI_RELU writes out = relu(acc +
-// bias); EPI_MASK (the data gradient of a 32 -> 32 layer through the ReLU
-// before it) writes out = acc where mask > 0, else 0.
-struct TcOut
-{
-	__nv_bfloat16 *out;
-	const __nv_bfloat16 *mask;
-};
-
+// EPI_RELU writes relu(acc + bias); EPI_MASK (the data gradient of a 32 -> 32
+// layer through the ReLU before it) writes acc where mask > 0, else 0.
 template <int EPI>
 __global__ void __launch_bounds__(tc::THREADS, 2) conv32_tc_kernel(const __grid_constant__ CUtensorMap tmap,
+                                                                    const __grid_constant__ CUtensorMap out_map,
                                                                     const __nv_bfloat16 *wt, const float *bias,
-                                                                    TcOut o, int n, int h, int w, uint32_t *err)
+                                                                    const __nv_bfloat16 *mask, int n, int h, int w,
+                                                                    uint32_t *err)
 {
 	using namespace pgs_umma;
 	extern __shared__ uint8_t smem_dyn[];
 	uint8_t *base = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~uintptr_t(1023));
-	uint8_t *sw = base + tc::STAGES * tc::STAGE_BYTES;
+	uint8_t *sw = base + tc::STAGES * tc::STAGE_BYTES, *sout = sw + tc::W_BYTES;
 	__shared__ uint64_t full_bar[tc::STAGES], empty_bar[tc::STAGES], acc_full[tc::ACCS], acc_empty[tc::ACCS];
 	__shared__ uint32_t tmem_slot;
-	__shared__ float s_bias[32];
+	__shared__ __align__(16) float s_bias[32];
 	__shared__ volatile uint32_t s_abort;
 
 	const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
@@ -776,7 +783,7 @@ __global__ void __launch_bounds__(tc::THREADS, 2) conv32_tc_kernel(const __grid_
 	if (tid < 32)
 		s_bias[tid] = EPI == EPI_MASK ? 0.0f : bias[tid];
 	if (warp == 0)
-		tmem_alloc(&tmem_slot, 64);
+		tmem_alloc(&tmem_slot, tc::ACCS * 32);
 	if (tid == 0)
 	{
 		for (int s = 0; s < tc::STAGES; s++)
@@ -815,28 +822,9 @@ __global__ void __launch_bounds__(tc::THREADS, 2) conv32_tc_kernel(const __grid_
 		if (lane == 0)
 		{
 			const uint32_t idesc = idesc_bf16_f32(128, 32);
-			int loaded = 0;
+			const uint64_t bd = smem_desc(smem_addr(sw), 16, 512, LAYOUT_SWIZZLE_64B);
 			for (int i = 0; i < mine && !s_abort; i++)
 			{
-				// Keep up to STAGES tiles of input in flight.
-				for (; loaded < mine && loaded < i + tc::STAGES; loaded++)
-				{
-					const int s = loaded % tc::STAGES;
-					if (loaded >= tc::STAGES && !mbar_wait_or_abort(&empty_bar[s], ((loaded / tc::STAGES) - 1) & 1, &s_abort))
-					{
-						atomicOr(err, 1u);
-						s_abort = 1;
-						break;
-					}
-					int img, x0, y0;
-					tile_coords(first + loaded * step, img, x0, y0);
-					uint8_t *dst = base + s * tc::STAGE_BYTES;
-					mbar_expect_tx(&full_bar[s], tc::STAGE_BYTES);
-					for (int dx = 0; dx < 3; dx++)
-						tma_load_4d(dst + dx * tc::COPY_BYTES, &tmap, &full_bar[s], 0, x0 - 1 + dx, y0 - 1, img);
-				}
-				if (s_abort)
-					break;
 				const int s = i % tc::STAGES, a = i % tc::ACCS;
 				if (!mbar_wait_or_abort(&full_bar[s], (i / tc::STAGES) & 1, &s_abort) ||
 				    (i >= tc::ACCS && !mbar_wait_or_abort(&acc_empty[a], ((i / tc::ACCS) - 1) & 1, &s_abort)))
@@ -846,24 +834,49 @@ __global__ void __launch_bounds__(tc::THREADS, 2) conv32_tc_kernel(const __grid_
 					break;
 				}
 				tc_fence_after();
-				const uint32_t a0 = smem_addr(base + s * tc::STAGE_BYTES), b0 = smem_addr(sw);
+				// Unrolled, with descriptors that differ from the first by constants
+				// (addresses in 16-byte units in the low bits): this one thread's
+				// instructions are what the tensor cores wait for otherwise.
+				const uint64_t ad = smem_desc(smem_addr(base + s * tc::STAGE_BYTES), 16, tc::ROW_BYTES, LAYOUT_SWIZZLE_64B);
 				const uint32_t d = tmem + uint32_t(a) * 32u;
-				bool acc = false;
+				#pragma unroll
 				for (int tap = 0; tap < 9; tap++)
 				{
 					const int dy = tap / 3, dx = tap % 3;
+					#pragma unroll
 					for (int ks = 0; ks < 2; ks++)
-					{
-						uint64_t ad = smem_desc(a0 + dx * tc::COPY_BYTES + dy * tc::COLS * 64u + ks * 32u, 16, 512,
-						                        LAYOUT_SWIZZLE_64B);
-						uint64_t bd = smem_desc(b0 + tap * 2048u + ks * 32u, 16, 512, LAYOUT_SWIZZLE_64B);
-						pgs_umma::mma_bf16(d, ad, bd, idesc, acc);
-						acc = true;
-					}
+						pgs_umma::mma_bf16(d, ad + ((dy * tc::ROW_BYTES + dx * 64u + ks * 32u) >> 4), bd + ((tap * 2048u + ks * 32u) >> 4),
+						                   idesc, tap + ks > 0);
 				}
 				mma_commit(&empty_bar[s]);
 				mma_commit(&acc_full[a]);
 			}
+		}
+		__syncwarp();
+	}
+	else if (warp == 5)
+	{
+		if (lane == 0)
+		{
+			int i = 0;
+			for (; i < mine && !s_abort; i++)
+			{
+				const int s = i % tc::STAGES;
+				if (i >= tc::STAGES && !mbar_wait_or_abort(&empty_bar[s], ((i / tc::STAGES) - 1) & 1, &s_abort))
+				{
+					atomicOr(err, 1u);
+					s_abort = 1;
+					break;
+				}
+				int img, x0, y0;
+				tile_coords(first + i * step, img, x0, y0);
+				mbar_expect_tx(&full_bar[s], tc::WIN_BYTES);
+				tma_load_4d(base + s * tc::STAGE_BYTES, &tmap, &full_bar[s], 0, x0 - 1, y0 - 1, img);
+			}
+			// Given up: the copies in flight still have to land.
+			if (s_abort)
+				for (int k = (i > tc::STAGES ? i - tc::STAGES : 0); k < i; k++)
+					mbar_wait_limit(&full_bar[k % tc::STAGES], (k / tc::STAGES) & 1, 1u << 20);
 		}
 		__syncwarp();
 	}
@@ -891,15 +904,13 @@ __global__ void __launch_bounds__(tc::THREADS, 2) conv32_tc_kernel(const __grid_
 				mbar_arrive(&acc_empty[a]);
 			int img, x0, y0;
 			tile_coords(first + i * step, img, x0, y0);
-			const int pix = int(quarter * 32u + lane);
-			const int gy = y0 + pix / tc::COLS, gx = x0 + pix % tc::COLS;
-			const size_t pixel = (size_t(img) * h + gy) * w + gx;
-			if (gx < w && gy < h)
+			uint32_t m[16] = {};
+			if (EPI == EPI_MASK)
 			{
-				uint32_t m[16];
-				if (EPI == EPI_MASK)
+				const int gy = y0 + int(quarter * 4u + lane / 8u), gx = x0 + int(lane % 8u);
+				if (gx < w && gy < h)
 				{
-					const uint4 *src = reinterpret_cast<const uint4 *>(o.mask + pixel * 32);
+					const uint4 *src = reinterpret_cast<const uint4 *>(mask + ((size_t(img) * h + gy) * w + gx) * 32);
 					#pragma unroll
 					for (int q = 0; q < 4; q++)
 					{
@@ -910,42 +921,60 @@ __global__ void __launch_bounds__(tc::THREADS, 2) conv32_tc_kernel(const __grid_
 						m[4 * q + 3] = t.w;
 					}
 				}
-				uint32_t packed[16];
-				#pragma unroll
-				for (int c = 0; c < 16; c++)
+			}
+			uint32_t packed[16];
+			#pragma unroll
+			for (int c = 0; c < 16; c++)
+			{
+				float lo, hi;
+				if (EPI == EPI_MASK)
 				{
-					float lo, hi;
-					if (EPI == EPI_MASK)
-					{
-						// Data gradient through the ReLU: keep where the layer's output was positive.
-						__nv_bfloat162 mk = *reinterpret_cast<const __nv_bfloat162 *>(&m[c]);
-						lo = __bfloat162float(mk.x) > 0.0f ? __uint_as_float(v[2 * c]) : 0.0f;
-						hi = __bfloat162float(mk.y) > 0.0f ? __uint_as_float(v[2 * c + 1]) : 0.0f;
-					}
-					else
-					{
-						lo = fmaxf(__uint_as_float(v[2 * c]) + s_bias[2 * c], 0.0f);
-						hi = fmaxf(__uint_as_float(v[2 * c + 1]) + s_bias[2 * c + 1], 0.0f);
-					}
-					packed[c] = pack_bf16x2(lo, hi);
+					// Data gradient through the ReLU: keep where the layer's output was positive.
+					__nv_bfloat162 mk = *reinterpret_cast<const __nv_bfloat162 *>(&m[c]);
+					lo = __bfloat162float(mk.x) > 0.0f ? __uint_as_float(v[2 * c]) : 0.0f;
+					hi = __bfloat162float(mk.y) > 0.0f ? __uint_as_float(v[2 * c + 1]) : 0.0f;
 				}
-				uint4 *dst = reinterpret_cast<uint4 *>(o.out + pixel * 32);
-				#pragma unroll
-				for (int q = 0; q < 4; q++)
-					dst[q] = make_uint4(packed[4 * q], packed[4 * q + 1], packed[4 * q + 2], packed[4 * q + 3]);
+				else
+				{
+					lo = fmaxf(__uint_as_float(v[2 * c]) + s_bias[2 * c], 0.0f);
+					hi = fmaxf(__uint_as_float(v[2 * c + 1]) + s_bias[2 * c + 1], 0.0f);
+				}
+				packed[c] = pack_bf16x2(lo, hi);
+			}
+			// The warp's other buffer may still be read by its last store, this
+			// one by none (waited for by the lane that issues them).
+			uint8_t *buf = sout + ((quarter * tc::OUT_BUFS + uint32_t(i) % tc::OUT_BUFS) * tc::OUT_BYTES);
+			if (lane == 0)
+				bulk_wait_read<tc::OUT_BUFS - 1>();
+			__syncwarp();
+			#pragma unroll
+			for (int q = 0; q < 4; q++)
+				*reinterpret_cast<uint4 *>(buf + swz64_offset(lane, uint32_t(q) * 8u)) =
+				    make_uint4(packed[4 * q], packed[4 * q + 1], packed[4 * q + 2], packed[4 * q + 3]);
+			fence_proxy_async();
+			__syncwarp();
+			if (lane == 0)
+			{
+				// A box that starts below the image is not stored.
+				if (y0 + int(quarter * 4u) < h)
+					tma_store_4d(&out_map, buf, 0, x0, y0 + int(quarter * 4u), img);
+				bulk_commit();
 			}
 		}
+		if (lane == 0)
+			bulk_wait_all();
+		__syncwarp();
 	}
 	tc_fence_before();
 	__syncthreads();
 	tc_fence_after();
 	if (warp == 0)
-		tmem_dealloc(tmem, 64);
+		tmem_dealloc(tmem, tc::ACCS * 32);
 }
 
 // Tensor map of an N x H x W x 32 BF16 activation tensor for conv32_tc_kernel:
-// boxes of 32 channels x 16 columns x 10 rows, 64-byte swizzle, zero fill.
-static int make_act_tmap(CUtensorMap *m, const void *ptr, int n, int h, int w)
+// boxes of 32 channels x cols x rows, 64-byte swizzle, zero fill.
+static int make_act_tmap(CUtensorMap *m, const void *ptr, int n, int h, int w, int cols, int rows)
 {
 	using Encode = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
 	                            const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
@@ -962,7 +991,7 @@ static int make_act_tmap(CUtensorMap *m, const void *ptr, int n, int h, int w)
 	}
 	cuuint64_t dims[4] = { 32, cuuint64_t(w), cuuint64_t(h), cuuint64_t(n) };
 	cuuint64_t strides[3] = { 64, cuuint64_t(w) * 64, cuuint64_t(h) * w * 64 };
-	cuuint32_t box[4] = { 32, uint32_t(tc::COLS), uint32_t(tc::WIN_ROWS), 1 };
+	cuuint32_t box[4] = { 32, uint32_t(cols), uint32_t(rows), 1 };
 	cuuint32_t estr[4] = { 1, 1, 1, 1 };
 	CUresult r = encode(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void *>(ptr), dims, strides, box, estr,
 	                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
@@ -999,28 +1028,35 @@ struct Upscaler
 	{
 		const void *ptr;
 		int n, h, w;
+		bool store;
 		CUtensorMap map;
 	};
-	TmapEntry tmaps[12] = {};
+	static constexpr int MAX_TMAPS = 24;
+	TmapEntry tmaps[MAX_TMAPS] = {};
 	int tmap_count = 0;
 
-	int act_tmap(const void *ptr, int n, int h, int w, CUtensorMap *&out)
+	// Map of the input windows, or of a warp's output boxes.
+	int act_tmap(const void *ptr, int n, int h, int w, bool store, CUtensorMap &out)
 	{
 		for (int i = 0; i < tmap_count; i++)
-			if (tmaps[i].ptr == ptr && tmaps[i].n == n && tmaps[i].h == h && tmaps[i].w == w)
+			if (tmaps[i].ptr == ptr && tmaps[i].n == n && tmaps[i].h == h && tmaps[i].w == w && tmaps[i].store == store)
 			{
-				out = &tmaps[i].map;
+				out = tmaps[i].map;
 				return PGS_OK;
 			}
-		TmapEntry &e = tmaps[tmap_count < 12 ? tmap_count++ : 11];
-		int r = make_act_tmap(&e.map, ptr, n, h, w);
+		TmapEntry &e = tmaps[tmap_count < MAX_TMAPS ? tmap_count++ : MAX_TMAPS - 1];
+		int r = store ? make_act_tmap(&e.map, ptr, n, h, w, tc::COLS, 4) : make_act_tmap(&e.map, ptr, n, h, w, tc::WIN_COLS, tc::WIN_ROWS);
 		if (r)
+		{
+			e.ptr = nullptr;
 			return r;
+		}
+		e.store = store;
 		e.ptr = ptr;
 		e.n = n;
 		e.h = h;
 		e.w = w;
-		out = &e.map;
+		out = e.map;
 		return PGS_OK;
 	}
 
@@ -1170,15 +1206,16 @@ struct Upscaler
 	template <int EPI>
 	int conv_tc(const ConvArgs &a, bool pdl = false)
 	{
-		CUtensorMap *m = nullptr;
-		int r = act_tmap(a.in, a.n, a.h, a.w, m);
+		CUtensorMap in, out;
+		int r = act_tmap(a.in, a.n, a.h, a.w, false, in);
+		if (!r)
+			r = act_tmap(a.out, a.n, a.h, a.w, true, out);
 		if (r)
 			return r;
 		int tiles = ((a.w + tc::COLS - 1) / tc::COLS) * ((a.h + tc::ROWS - 1) / tc::ROWS) * a.n;
 		int grid = std::min(tiles, sm_count * use_tc);
-		TcOut o = { a.out, a.mask };
-		return launch(conv32_tc_kernel<EPI>, dim3(grid), dim3(tc::THREADS), tc::SMEM_BYTES, pdl, *m, a.wt, a.bias, o,
-		              a.n, a.h, a.w, d_err);
+		return launch(conv32_tc_kernel<EPI>, dim3(grid), dim3(tc::THREADS), tc::SMEM_BYTES, pdl, in, out, a.wt, a.bias,
+		              a.mask, a.n, a.h, a.w, d_err);
 	}
 
 	template <int CIN, int COUT, int EPI>
