@@ -226,17 +226,22 @@ static void build_phase_lut(uint32_t rx, uint32_t ry, uint32_t *lut)
 
 // Level 0 sampling constants of one axis (TexAxis): `mode` keeps only the
 // region wrap modes, plain REPEAT and CLAMP come from the primitive's bit.
-static TexAxis sampler_axis(uint32_t mode, bool clamp, uint32_t size_log2, uint32_t lo, uint32_t hi, uint32_t place)
+static TexAxis sampler_axis(bool perspective, bool clamp, uint32_t mode, uint32_t size_log2, uint32_t lo, uint32_t hi,
+                            uint32_t place)
 {
 	if (mode < WRAP_REGION_CLAMP)
 		mode = clamp ? WRAP_CLAMP : WRAP_REPEAT;
 	const WrapAxis w = wrap_axis(mode, size_log2, lo, hi);
-	TexAxis a = { w.and_mask, w.or_mask, w.lo, w.hi, -INFINITY, INFINITY, 16.0f * float(1u << size_log2), place };
+	const float scale = perspective ? 16.0f * float(1u << size_log2) : 16.0f;
+	TexAxis a = { w.and_mask, w.or_mask, w.lo, w.hi, -2047.0f * scale, 2047.0f * scale, scale, place };
 	if (clamp)
 	{
 		const bool region = mode == WRAP_REGION_CLAMP;
-		a.clamp_lo = 16.0f * (float(region ? lo : 0u) + 0.5f);
-		a.clamp_hi = 16.0f * (float(region ? hi : (1u << size_log2) - 1u) + 0.5f);
+		const float first = 16.0f * (float(region ? lo : 0u) + 0.5f);
+		const float last = 16.0f * (float(region ? hi : (1u << size_log2) - 1u) + 0.5f);
+		// min(max(x, first), last) of x within the bounds so far.
+		a.clamp_lo = std::min(std::max(a.clamp_lo, first), last);
+		a.clamp_hi = std::min(std::max(a.clamp_hi, first), last);
 	}
 	return a;
 }
@@ -784,10 +789,10 @@ struct CudaBackend
 					max_texels = std::max(max_texels, n);
 				}
 				const TexImage &base_image = im[i * TEX_SLOTS];
-				for (uint32_t clamp = 0; clamp < 2; clamp++)
+				for (uint32_t way = 0; way < 4; way++)
 				{
-					smp[i].u[clamp] = sampler_axis(t.wms, clamp, t.tw_log2, t.minu, t.maxu, base_image.offset);
-					smp[i].v[clamp] = sampler_axis(t.wmt, clamp, t.th_log2, t.minv, t.maxv, base_image.ext_u);
+					smp[i].u[way] = sampler_axis(way & 2u, way & 1u, t.wms, t.tw_log2, t.minu, t.maxu, base_image.offset);
+					smp[i].v[way] = sampler_axis(way & 2u, way & 1u, t.wmt, t.th_log2, t.minv, t.maxv, base_image.ext_u);
 				}
 			}
 			if (texels > (uint64_t(1) << 31))

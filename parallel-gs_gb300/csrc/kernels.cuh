@@ -112,10 +112,10 @@ struct TexImage
 };
 
 // How level 0 of a texture is sampled along one axis: a wrap mode as
-// (v & and_mask | or_mask) clamped to [lo, hi], the coordinate clamp of the
-// sampler (infinite bounds where it has none) in 1/16 texels, and 16 x the
-// texture size for perspective coordinates.  `place` is the image's first texel
-// on the U axis and its row length on the V axis.
+// (v & and_mask | or_mask) clamped to [lo, hi], the scale to 1/16 texels, and
+// the bounds of the coordinate there (the +-2047 of every coordinate and the
+// sampler's own clamp).  `place` is the image's first texel on the U axis and
+// its row length on the V axis.
 struct __align__(16) TexAxis
 {
 	int32_t and_mask, or_mask, lo, hi;
@@ -123,10 +123,11 @@ struct __align__(16) TexAxis
 	uint32_t place;
 };
 
-// Both axes, each without and with the primitive's clamp bit.
+// Both axes, for texel and perspective coordinates (+ 2), each without and with
+// the primitive's clamp bit (+ 1).
 struct TexSampler
 {
-	TexAxis u[2], v[2];
+	TexAxis u[4], v[4];
 };
 
 // Flat-primitive depth buckets found by triangle setup in a super-sampled pass
@@ -1466,15 +1467,17 @@ __device__ void sample_level(const PassParams &P, uint32_t tex_index, const pgs_
 }
 
 // Level 0 of a texture, from the constants of its sampler record: the same
-// texels as sample_level with level 0 (scaling by 16 x a power of two is exact,
-// and a coordinate of a sampler without clamping has infinite bounds).
+// texels as sample_level with level 0 and coordinates clamped to +-2047 before
+// (scaling by a power of two is exact, so the clamps commute with it).
 __device__ __forceinline__ void sample_base(const PassParams &P, uint32_t tex_index, uint32_t tex_word, float u, float v,
                                             bool perspective, uint32_t rgba[4])
 {
 	const TexSampler &T = P.samplers[tex_index];
-	const TexAxis au = T.u[(tex_word & TEX_SAMPLER_CLAMP_S_BIT) ? 1 : 0], av = T.v[(tex_word & TEX_SAMPLER_CLAMP_T_BIT) ? 1 : 0];
-	const float u16 = fminf(fmaxf(fmul(u, perspective ? au.scale : 16.0f), au.clamp_lo), au.clamp_hi);
-	const float v16 = fminf(fmaxf(fmul(v, perspective ? av.scale : 16.0f), av.clamp_lo), av.clamp_hi);
+	const uint32_t way = perspective ? 2u : 0u;
+	const TexAxis au = T.u[way + ((tex_word & TEX_SAMPLER_CLAMP_S_BIT) ? 1u : 0u)];
+	const TexAxis av = T.v[way + ((tex_word & TEX_SAMPLER_CLAMP_T_BIT) ? 1u : 0u)];
+	const float u16 = fminf(fmaxf(fmul(u, au.scale), au.clamp_lo), au.clamp_hi);
+	const float v16 = fminf(fmaxf(fmul(v, av.scale), av.clamp_lo), av.clamp_hi);
 	const int32_t ku = __float2int_rd(fadd(u16, 1.0f / 64.0f)), kv = __float2int_rd(fadd(v16, 1.0f / 64.0f));
 	const uint32_t *img = P.texels + au.place;
 	const WrapAxis wu = { au.and_mask, au.or_mask, au.lo, au.hi }, wv = { av.and_mask, av.or_mask, av.lo, av.hi };
@@ -1711,8 +1714,12 @@ __device__ __forceinline__ void combined_color(const ShadeCtx &C, uint32_t pi, c
 			s = __fdiv_rn(s, q);
 			t = __fdiv_rn(t, q);
 		}
-		s = fminf(fmaxf(s, -2047.0f), 2047.0f);
-		t = fminf(fmaxf(t, -2047.0f), 2047.0f);
+		if (MIP)
+		{
+			// (sample_base's bounds include these.)
+			s = fminf(fmaxf(s, -2047.0f), 2047.0f);
+			t = fminf(fmaxf(t, -2047.0f), 2047.0f);
+		}
 		float tx[4];
 		sample_texture<MIP>(P, tex, tex2, s, t, q, perspective, C.sample,
 		                    C.ss ? C.I->rate_x_log2 : 0u, C.ss ? C.I->rate_y_log2 : 0u, tx);
@@ -1769,7 +1776,7 @@ struct SampleState
 	uint32_t pending_prim;
 };
 
-template <bool MIP>
+template <bool MIP, bool AA>
 __device__ __forceinline__ void shade_resolve(const ShadeCtx &C, SampleState &S, uint32_t pi, const Request &r)
 {
 	const PassParams &P = *C.P;
@@ -1791,7 +1798,7 @@ __device__ __forceinline__ void shade_resolve(const ShadeCtx &C, SampleState &S,
 	const uint32_t bm = sv.y;
 	bool abe = (bm & BLEND_MODE_ABE_BIT) != 0;
 
-	if (P.has_aa1)
+	if (AA && P.has_aa1)
 	{
 		const bool multisample = (pst >> STATE_BIT_MULTISAMPLE) & 1;
 		bool use_cov = (cc[3] == 128.0f || !abe) && multisample;
@@ -2130,7 +2137,7 @@ __device__ __forceinline__ void process_primitive_with(const ShadeCtx &C, uint32
 		if (__any_sync(0xffffffffu, q.coverage > 0 && S.pending.coverage > 0))
 		{
 			if (S.pending.coverage > 0)
-				shade_resolve<MIP>(C, S, S.pending_prim, S.pending);
+				shade_resolve<MIP, AA>(C, S, S.pending_prim, S.pending);
 			S.pending.coverage = 0;
 			S.pending.z_write = false;
 		}
@@ -2140,7 +2147,7 @@ __device__ __forceinline__ void process_primitive_with(const ShadeCtx &C, uint32
 			{
 				S.pending = q;
 				S.pending_prim = pi;
-				shade_resolve<MIP>(C, S, S.pending_prim, S.pending);
+				shade_resolve<MIP, AA>(C, S, S.pending_prim, S.pending);
 				S.pending.coverage = 0;
 				S.pending.z_write = false;
 			}
@@ -2193,7 +2200,7 @@ __device__ __forceinline__ void process_primitive_with(const ShadeCtx &C, uint32
 	if (__any_sync(0xffffffffu, need_flush))
 	{
 		if (S.pending.coverage > 0)
-			shade_resolve<MIP>(C, S, S.pending_prim, S.pending);
+			shade_resolve<MIP, AA>(C, S, S.pending_prim, S.pending);
 		S.pending.coverage = 0;
 		S.pending.z_write = false;
 		if (q.coverage > 0)
@@ -2208,7 +2215,7 @@ __device__ __forceinline__ void process_primitive_with(const ShadeCtx &C, uint32
 	{
 		if (S.pending.coverage > 0 && S.pending_prim == pi)
 		{
-			shade_resolve<MIP>(C, S, S.pending_prim, S.pending);
+			shade_resolve<MIP, AA>(C, S, S.pending_prim, S.pending);
 			S.pending.coverage = 0;
 			S.pending.z_write = false;
 		}
@@ -2581,7 +2588,7 @@ __device__ __forceinline__ void walk_batch(const ShadeCtx &C, const uint32_t *id
 		else
 			break;
 		if (act)
-			shade_resolve<false>(C, S, rp, r);
+			shade_resolve<false, false>(C, S, rp, r);
 		__syncwarp();
 	}
 }
@@ -2626,13 +2633,24 @@ __device__ __forceinline__ ListScan list_scan(const DevInstance &I, const uint32
 {
 	const unsigned full = 0xffffffffu;
 	const uint32_t lane = threadIdx.x & 31u, SW = I.summary_words;
-	for (uint32_t sw = threadIdx.x >> 5; sw < SW; sw += WARPS)
+	// Four words at a time, so that their loads are in flight together.
+	for (uint32_t sw = threadIdx.x >> 5; sw < SW; sw += 4u * WARPS)
 	{
-		const uint32_t words = __ldg(summary + sw);
-		const uint32_t mw = ((words >> lane) & 1u) ? __ldg(mask + sw * 32u + lane) : 0u;
-		const uint32_t c = __reduce_add_sync(full, uint32_t(__popc(mw)));
-		if (lane == 0)
-			L.count[sw] = c;
+		uint32_t words[4], mw[4];
+		#pragma unroll
+		for (int k = 0; k < 4; k++)
+			words[k] = sw + k * WARPS < SW ? __ldg(summary + sw + k * WARPS) : 0u;
+		#pragma unroll
+		for (int k = 0; k < 4; k++)
+			mw[k] = ((words[k] >> lane) & 1u) ? __ldg(mask + (sw + k * WARPS) * 32u + lane) : 0u;
+		#pragma unroll
+		for (int k = 0; k < 4; k++)
+			if (sw + k * WARPS < SW)
+			{
+				const uint32_t c = __reduce_add_sync(full, uint32_t(__popc(mw[k])));
+				if (lane == 0)
+					L.count[sw + k * WARPS] = c;
+			}
 	}
 	__syncthreads();
 	ListScan r;
@@ -2904,7 +2922,7 @@ __device__ __forceinline__ void shade_subtile(const PassParams &P, const DevInst
 
 	// walk_batch leaves nothing pending.
 	if ((AA || !CULL) && S.pending.coverage > 0)
-		shade_resolve<MIP>(C, S, S.pending_prim, S.pending);
+		shade_resolve<MIP, AA>(C, S, S.pending_prim, S.pending);
 
 	// Covered-sample counter: one atomic per warp.
 	{
