@@ -1087,20 +1087,20 @@ struct CudaBackend
 	// gs/gs_renderer.cpp:2395-2415).
 	template <bool AA, bool MIP>
 	void launch_shade(const PassParams &P, const DevInstance &I, uint32_t ns_log2, uint32_t grid,
-	                  const uint32_t *masks, const uint32_t *summary, const uint32_t *d_flags)
+	                  const uint32_t *masks, const uint32_t *d_flags)
 	{
 		if (I.rate_y_log2 != 0)
 		{
 			switch (ns_log2)
 			{
-			case 1: shade_kernel<2, true, AA, MIP><<<grid * ShadeCta<2>::PARTS, ShadeCta<2>::THREADS, 0, stream>>>(P, I, masks, summary, d_flags); break;
-			case 2: shade_kernel<4, true, AA, MIP><<<grid * ShadeCta<4>::PARTS, ShadeCta<4>::THREADS, 0, stream>>>(P, I, masks, summary, d_flags); break;
-			case 3: shade_kernel<8, true, AA, MIP><<<grid * ShadeCta<8>::PARTS, ShadeCta<8>::THREADS, 0, stream>>>(P, I, masks, summary, d_flags); break;
-			default: shade_kernel<16, true, AA, MIP><<<grid * ShadeCta<16>::PARTS, ShadeCta<16>::THREADS, 0, stream>>>(P, I, masks, summary, d_flags); break;
+			case 1: shade_kernel<2, true, AA, MIP><<<grid * ShadeCta<2>::PARTS, ShadeCta<2>::THREADS, 0, stream>>>(P, I, masks, d_flags); break;
+			case 2: shade_kernel<4, true, AA, MIP><<<grid * ShadeCta<4>::PARTS, ShadeCta<4>::THREADS, 0, stream>>>(P, I, masks, d_flags); break;
+			case 3: shade_kernel<8, true, AA, MIP><<<grid * ShadeCta<8>::PARTS, ShadeCta<8>::THREADS, 0, stream>>>(P, I, masks, d_flags); break;
+			default: shade_kernel<16, true, AA, MIP><<<grid * ShadeCta<16>::PARTS, ShadeCta<16>::THREADS, 0, stream>>>(P, I, masks, d_flags); break;
 			}
 			launch_counter++;
 		}
-		shade_kernel<1, false, AA, MIP><<<grid, 64, 0, stream>>>(P, I, masks, summary, d_flags);
+		shade_kernel<1, false, AA, MIP><<<grid, 64, 0, stream>>>(P, I, masks, d_flags);
 		launch_counter++;
 	}
 
@@ -1136,7 +1136,6 @@ struct CudaBackend
 		I.prim_lo = lo;
 		I.prim_count = count;
 		I.mask_words = (count + 31) / 32;
-		I.summary_words = (I.mask_words + 31) / 32;
 		I.sub_w = I.tiles_w << (p.tile_size_log2 - 3);
 		I.sub_h = I.tiles_h << (p.tile_size_log2 - 3);
 		size_t tiles = size_t(I.tiles_w) * I.tiles_h;
@@ -1149,18 +1148,18 @@ struct CudaBackend
 		// Super-sampled shading touches planes 1 .. 1 + 2^ns_log2.
 		if (I.rate_y_log2 != 0 && 2u + (1u << ns_log2) > num_planes)
 			return PGS_ERROR_INVALID_ARGUMENT;
-		size_t mask_words = subs * I.mask_words, summary_words = subs * I.summary_words;
-		// Sub-tile masks, their summaries and the coarse tiles' flags, cleared together.
-		int r = ensure_masks(mask_words + summary_words + tiles);
+		size_t mask_words = subs * I.mask_words;
+		// Sub-tile masks and the coarse tiles' flags, cleared together.
+		int r = ensure_masks(mask_words + tiles);
 		if (r)
 			return r;
-		uint32_t *d_sub_masks = d_masks, *d_sub_summary = d_masks + mask_words, *d_flags = d_sub_summary + summary_words;
+		uint32_t *d_flags = d_masks + mask_words;
 		{
 			StageScope ts(this, PGS_TIMESTAMP_BINNING);
-			CUDA_TRY(cudaMemsetAsync(d_masks, 0, (mask_words + summary_words + tiles) * sizeof(uint32_t), stream));
+			CUDA_TRY(cudaMemsetAsync(d_masks, 0, (mask_words + tiles) * sizeof(uint32_t), stream));
 			// A pass of few primitives spreads each group's candidates over more CTAs.
 			const uint32_t groups = (count + 31) / 32, slices = std::min(std::max(BIN_TARGET_CTAS / groups, 1u), 16u);
-			bin_kernel<<<dim3(groups, slices), 32 * BIN_GROUP_WARPS, 0, stream>>>(P, I, d_sub_masks, d_sub_summary, d_flags);
+			bin_kernel<<<dim3(groups, slices), 32 * BIN_GROUP_WARPS, 0, stream>>>(P, I, d_masks, d_flags);
 			launch_counter++;
 		}
 		uint32_t grid = uint32_t(subs);
@@ -1169,12 +1168,11 @@ struct CudaBackend
 		{
 			collect->P = P;
 			collect->I = I;
-			collect->masks = d_sub_masks;
-			collect->summary = d_sub_summary;
+			collect->masks = d_masks;
 			collect->flags = d_flags;
 			collect->ns_log2 = I.rate_y_log2 != 0 ? ns_log2 : 0u;
 			collect->aa = p.has_aa1;
-			collect->units = uint32_t(subs) * (2u << collect->ns_log2);
+			collect->units = uint32_t(subs) << collect->ns_log2; // of 64 samples
 			*collected = true;
 			CUDA_TRY(cudaGetLastError());
 			return PGS_OK;
@@ -1190,11 +1188,11 @@ struct CudaBackend
 		// variant too (three variants per rate).
 		StageScope ts(this, PGS_TIMESTAMP_SHADING);
 		if (p.has_mipmap || p.has_ss_textures)
-			launch_shade<true, true>(P, I, ns_log2, grid, d_sub_masks, d_sub_summary, d_flags);
+			launch_shade<true, true>(P, I, ns_log2, grid, d_masks, d_flags);
 		else if (p.has_aa1)
-			launch_shade<true, false>(P, I, ns_log2, grid, d_sub_masks, d_sub_summary, d_flags);
+			launch_shade<true, false>(P, I, ns_log2, grid, d_masks, d_flags);
 		else
-			launch_shade<false, false>(P, I, ns_log2, grid, d_sub_masks, d_sub_summary, d_flags);
+			launch_shade<false, false>(P, I, ns_log2, grid, d_masks, d_flags);
 		CUDA_TRY(cudaGetLastError());
 		if (shade_timing)
 			return record_timing_event(shade_ev[1]);
@@ -2294,7 +2292,7 @@ struct BatchEngine
 	int launch(size_t first, size_t count, uint32_t units, uint32_t counter)
 	{
 		uint32_t grid = std::max<uint32_t>(1u, std::min<uint32_t>(uint32_t(sm_count) * ctas_per_sm,
-		                                                          (units + BLOCK / 32 - 1) / (BLOCK / 32)));
+		                                                          units));
 		batch_shade_kernel<BLOCK><<<grid, BLOCK, 0, master>>>(d_items + first, uint32_t(count), units,
 		                                                      d_counters + counter);
 		CUDA_TRY(cudaGetLastError());
@@ -2424,7 +2422,7 @@ struct BatchEngine
 						for (ShadeItem &x : round_items)
 						{
 							x.unit_base = units;
-							units += x.units;
+							units += (x.units * 64u + block - 1u) / block;
 						}
 						ShadeItem *it = h_items + first;
 						memcpy(it, round_items.data(), count * sizeof(ShadeItem));

@@ -64,7 +64,6 @@ struct DevInstance
 	uint32_t instance;
 	uint32_t prim_lo, prim_count; // primitive range of this dispatch
 	uint32_t mask_words;          // bitmask words per 8x8 sub-tile (1 bit per primitive)
-	uint32_t summary_words;       // summary words per sub-tile (1 bit per mask word)
 	uint32_t sub_w, sub_h;        // 8x8 sub-tiles per row / column
 	int32_t snap_mask_y;          // raster snap of rows: half the sample pitch when field rendering
 	uint32_t force_ss;            // field rendering: every covered tile super-sampled
@@ -983,8 +982,8 @@ __device__ __forceinline__ bool intersects_tile(const PrimSetup &s, int32_t lo0,
 // K2: binning.  Coarse tiles (2^tile_size_log2 pixels) carry the reference's
 // membership test and super-sampling flags (binning.comp:74-125); shading
 // lists are kept per 8x8 sub-tile as bitmasks over the pass's primitive range
-// so that ascending primitive order needs no sort.  A summary bitmask marks
-// non-empty mask words.  The primitives of one mask word (32) are a group; its
+// so that ascending primitive order needs no sort.  The primitives of one mask
+// word (32) are a group; its
 // (primitive, tile) candidates, those of the coarse grid and then those of the
 // sub-tile grid, are dealt out 32 at a time to the warps of gridDim.y CTAs, so
 // that neither a primitive over the whole frame nor one over hundreds of coarse
@@ -1050,7 +1049,7 @@ __device__ __forceinline__ void deal_tiles(const BinItem *items, uint32_t n, int
 }
 
 __global__ void __launch_bounds__(32 * BIN_GROUP_WARPS) bin_kernel(PassParams P, DevInstance I, uint32_t *sub_masks,
-                                                                   uint32_t *sub_summary, uint32_t *tile_flags)
+                                                                   uint32_t *tile_flags)
 {
 	__shared__ BinItem items[32];
 	__shared__ uint32_t s_n;
@@ -1115,12 +1114,9 @@ __global__ void __launch_bounds__(32 * BIN_GROUP_WARPS) bin_kernel(PassParams P,
 		const int32_t sx = I.base_x + (gx << 3), sy = I.base_y + (gy << 3);
 		if (!intersects_tile(it.s, sx, sy, sx + 7, sy + 7, it.ms_tri))
 			return;
-		// Results unused: both compile to fire-and-forget reductions.
-		const uint32_t word = it.local >> 5, bit = 1u << (it.local & 31u);
-		const uint32_t sword = word >> 5, sbit = 1u << (word & 31u);
+		// Result unused: a fire-and-forget reduction.
 		const size_t sub = size_t(gy) * I.sub_w + size_t(gx);
-		atomicOr(&sub_masks[sub * I.mask_words + word], bit);
-		atomicOr(&sub_summary[sub * I.summary_words + sword], sbit);
+		atomicOr(&sub_masks[sub * I.mask_words + (it.local >> 5)], 1u << (it.local & 31u));
 		if (ts == 3)
 			mark_tile(it, uint32_t(sub));
 	});
@@ -1917,27 +1913,6 @@ __device__ __forceinline__ void shade_resolve(const ShadeCtx &C, SampleState &S,
 	}
 }
 
-// Coverage of one sample for primitives without AA1 (evaluate_coverage with
-// multisample == false): 0x80 when the sample is inside, else 0.  The
-// barycentrics are computed separately, only once some lane is covered.
-__device__ __forceinline__ int coverage_plain(const PrimSetup &s, int32_t cx, int32_t cy, int dim)
-{
-	int32_t sx = cx >> dim, sy = cy >> dim;
-	if (!(sx >= s.bb[0] && sy >= s.bb[1] && s.bb[2] >= sx && s.bb[3] >= sy))
-		return 0;
-	int32_t axw = s.a[0];
-	int32_t A[3] = { axw >> 6, s.a[1], s.a[2] };
-	int32_t px = cx << (3 - dim), py = cy << (3 - dim);
-	int32_t ea = idot3(A, px, py), eb = idot3(s.b, px, py), ec = idot3(s.c, px, py);
-	if ((axw & 1) && ea < 0)
-	{
-		eb += ea + int32_t((uint32_t(axw) >> 2) & 3u) - 1;
-		ec += ea + int32_t((uint32_t(axw) >> 4) & 3u) - 1;
-		ea = 0;
-	}
-	return (ea >= 0 && eb >= 0 && ec >= 0) ? 0x80 : 0;
-}
-
 __device__ __forceinline__ int evaluate_coverage(const PrimSetup &s, int32_t cx, int32_t cy, float &i, float &j, bool ms,
                                                  bool line, int dim)
 {
@@ -1992,9 +1967,9 @@ __device__ __forceinline__ int evaluate_coverage(const PrimSetup &s, int32_t cx,
 }
 
 // Must be called by all lanes of a warp; returns with warp_any == false (and no
-// further work) when no lane of the warp is covered.  AA compiles the AA1
-// coverage path in (ubershader variant VARIANT_FLAG_HAS_AA1_BIT).
-template <bool AA, bool TEX_ARRAY>
+// further work) when no lane of the warp is covered.  The AA1 variants' path
+// (ubershader variant VARIANT_FLAG_HAS_AA1_BIT); the others go by coverage masks.
+template <bool TEX_ARRAY>
 __device__ __forceinline__ Request shade_early(const ShadeCtx &C, const PrimSetup &s, uint32_t pi, uint32_t st,
                                                const SampleState &S, bool &opaque, bool &warp_any)
 {
@@ -2003,7 +1978,7 @@ __device__ __forceinline__ Request shade_early(const ShadeCtx &C, const PrimSetu
 	opaque = (st >> STATE_BIT_OPAQUE) & 1;
 	r.z_test = C.zs && ((st >> STATE_BIT_Z_TEST) & 1);
 	r.z_write = C.zs && ((st >> STATE_BIT_Z_WRITE) & 1);
-	const bool multisample = AA && ((st >> STATE_BIT_MULTISAMPLE) & 1);
+	const bool multisample = (st >> STATE_BIT_MULTISAMPLE) & 1;
 	int32_t rx = S.hx, ry = S.hy;
 	if (C.ss && (st & (1u << STATE_BIT_SNAP_RASTER)))
 	{
@@ -2013,10 +1988,7 @@ __device__ __forceinline__ Request shade_early(const ShadeCtx &C, const PrimSetu
 		ry &= (TEX_ARRAY && (P.prims[pi].tex & TEX_SAMPLE_MAPPING_BIT)) ? C.snap_mask_x : C.snap_mask_y;
 	}
 	float i = 0.0f, j = 0.0f;
-	if (AA)
-		r.coverage = evaluate_coverage(s, rx, ry, i, j, multisample, (st >> STATE_BIT_LINE) & 1, C.dim);
-	else
-		r.coverage = coverage_plain(s, rx, ry, C.dim);
+	r.coverage = evaluate_coverage(s, rx, ry, i, j, multisample, (st >> STATE_BIT_LINE) & 1, C.dim);
 	if (P.has_scanmsk)
 	{
 		int32_t sy = S.hy;
@@ -2028,13 +2000,6 @@ __device__ __forceinline__ Request shade_early(const ShadeCtx &C, const PrimSetu
 	warp_any = __any_sync(0xffffffffu, r.coverage > 0);
 	if (!warp_any)
 		return r;
-	if (!AA)
-	{
-		// Barycentrics at the raster coordinate (evaluate_coverage_single).
-		int32_t qx = rx << (3 - C.dim), qy = ry << (3 - C.dim);
-		i = fadd(fmul(__int2float_rn(idot3(s.b, qx, qy)), s.inv_area), s.error_i);
-		j = fadd(fmul(__int2float_rn(idot3(s.c, qx, qy)), s.inv_area), s.error_j);
-	}
 	if (C.zs && multisample && r.coverage < 0x80)
 		r.z_write = false;
 	uint32_t z = s.z[0];
@@ -2101,12 +2066,12 @@ __device__ __forceinline__ void sample_offset(uint32_t s, uint32_t xl, uint32_t 
 // (primitive_intersects_tile); a second test against each warp's smaller
 // rectangle costs more than the coverage test it would skip, so coverage
 // alone decides.
-template <bool SS, bool AA, bool MIP>
+template <bool SS, bool MIP>
 __device__ __forceinline__ void process_primitive_with(const ShadeCtx &C, uint32_t pi, const PrimSetup &s, uint32_t st,
                                                        SampleState &S, uint32_t &covered)
 {
 	bool opaque, any_cov;
-	Request q = shade_early<AA, MIP>(C, s, pi, st, S, opaque, any_cov);
+	Request q = shade_early<MIP>(C, s, pi, st, S, opaque, any_cov);
 	if (!any_cov)
 		return;
 	// A primitive that is not opaque (warp-uniform: a state bit) is shaded
@@ -2137,7 +2102,7 @@ __device__ __forceinline__ void process_primitive_with(const ShadeCtx &C, uint32
 		if (__any_sync(0xffffffffu, q.coverage > 0 && S.pending.coverage > 0))
 		{
 			if (S.pending.coverage > 0)
-				shade_resolve<MIP, AA>(C, S, S.pending_prim, S.pending);
+				shade_resolve<MIP, true>(C, S, S.pending_prim, S.pending);
 			S.pending.coverage = 0;
 			S.pending.z_write = false;
 		}
@@ -2147,7 +2112,7 @@ __device__ __forceinline__ void process_primitive_with(const ShadeCtx &C, uint32
 			{
 				S.pending = q;
 				S.pending_prim = pi;
-				shade_resolve<MIP, AA>(C, S, S.pending_prim, S.pending);
+				shade_resolve<MIP, true>(C, S, S.pending_prim, S.pending);
 				S.pending.coverage = 0;
 				S.pending.z_write = false;
 			}
@@ -2200,7 +2165,7 @@ __device__ __forceinline__ void process_primitive_with(const ShadeCtx &C, uint32
 	if (__any_sync(0xffffffffu, need_flush))
 	{
 		if (S.pending.coverage > 0)
-			shade_resolve<MIP, AA>(C, S, S.pending_prim, S.pending);
+			shade_resolve<MIP, true>(C, S, S.pending_prim, S.pending);
 		S.pending.coverage = 0;
 		S.pending.z_write = false;
 		if (q.coverage > 0)
@@ -2215,19 +2180,19 @@ __device__ __forceinline__ void process_primitive_with(const ShadeCtx &C, uint32
 	{
 		if (S.pending.coverage > 0 && S.pending_prim == pi)
 		{
-			shade_resolve<MIP, AA>(C, S, S.pending_prim, S.pending);
+			shade_resolve<MIP, true>(C, S, S.pending_prim, S.pending);
 			S.pending.coverage = 0;
 			S.pending.z_write = false;
 		}
 	}
 }
 
-template <bool SS, bool AA, bool MIP>
+template <bool SS, bool MIP>
 __device__ __forceinline__ void process_primitive(const ShadeCtx &C, uint32_t pi, SampleState &S, uint32_t &covered)
 {
 	const PassParams &P = *C.P;
 	const PrimSetup s = P.setup[pi];
-	process_primitive_with<SS, AA, MIP>(C, pi, s, P.prims[pi].state, S, covered);
+	process_primitive_with<SS, MIP>(C, pi, s, P.prims[pi].state, S, covered);
 }
 
 // ---------------------------------------------------------------------------
@@ -2256,12 +2221,11 @@ __device__ __forceinline__ bool edge_may_pass(const int32_t e[3], int4 r, int sh
 // position lies in r = (x0, y0, x1, y1).  Parallelograms (sprites, lines,
 // fused rectangles) shift edges past the diagonal and AA1 multisampled
 // edges cover outside the triangle, so those keep to the box test.
-template <bool AA>
 __device__ __forceinline__ bool may_cover(const PrimSetup &s, uint32_t st, int4 r, int dim)
 {
 	if ((r.z >> dim) < s.bb[0] || (r.x >> dim) > s.bb[2] || (r.w >> dim) < s.bb[1] || (r.y >> dim) > s.bb[3])
 		return false;
-	if (((st >> STATE_BIT_PARALLELOGRAM) & 1u) || (AA && ((st >> STATE_BIT_MULTISAMPLE) & 1u)))
+	if (((st >> STATE_BIT_PARALLELOGRAM) & 1u) || ((st >> STATE_BIT_MULTISAMPLE) & 1u))
 		return true;
 	const int sh = 3 - dim;
 	const int32_t A[3] = { s.a[0] >> 6, s.a[1], s.a[2] };
@@ -2606,83 +2570,105 @@ struct ShadeCta
 	static constexpr uint32_t WARPS = THREADS / 32u;
 };
 
-// The sub-tile's primitive list, expanded by the whole CTA into primitive
-// indices in ascending order in shared memory (CAP at a time), then walked by
-// each warp on its own, 32 primitives at a time.  Expansion: each warp counts
-// the primitives under its summary words, every warp turns the counts into
-// offsets, and each writes the indices under its words at those offsets.
-constexpr uint32_t LIST_CAP = 2048u;
-// One summary word per 32 mask words of 32 primitives.
-constexpr uint32_t LIST_MAX_SW = (PGS_MAX_PRIMITIVES_PER_FLUSH + 1023u) / 1024u;
-static_assert(LIST_MAX_SW <= 64, "list_scan holds two offsets per lane");
+// The sub-tile's primitive list, expanded by the T threads that shade it
+// together into primitive indices in ascending order in shared memory (CAP at a
+// time), then walked by each warp on its own, 32 primitives at a time.  Each
+// thread takes LIST_WORDS mask words of a chunk of T * LIST_WORDS, all loads in
+// flight at once, keeps them in registers, and writes the indices of their bits
+// where a scan over the threads puts them.
+// Bound: latency of the loads and barriers; most of a sub-tile's words are empty.
+// A summary bitmask over the words, read first, saved reads of empty words but
+// cost a round trip, and binning a second reduction per pair: plain frame of
+// 10,000 primitives 48.6 us with it, 45.5 without; textured 4x frame of 52,000
+// primitives 596 and 580 us (binning 45 and 37 of them).
+constexpr uint32_t LIST_WORDS = 4;
 
+template <uint32_t T, uint32_t CAP>
 struct ListShared
 {
-	uint32_t ids[LIST_CAP];
-	uint32_t count[LIST_MAX_SW];
+	uint32_t ids[CAP];
+	uint32_t count[LIST_WORDS * T / 32u]; // per word of the chunk and warp
+	int2 smp[16];                         // sample offsets of WarpPlace
+	int4 rect[T / 32u];                   // per warp, AA1 variants
 };
 
-// Offsets of summary words `lane` and `lane + 32` in the list, and its length.
-struct ListScan
+// The T threads that run a sub-tile together: thread 0 of them is aligned to T,
+// and `bar` is a barrier of their own (0 where they are the whole CTA).
+template <uint32_t T>
+struct ShadeGroup
 {
-	uint32_t lo, hi, total;
+	uint32_t bar;
+	__device__ __forceinline__ uint32_t thread() const { return threadIdx.x & (T - 1u); }
+	__device__ __forceinline__ void sync() const { asm volatile("bar.sync %0, %1;" ::"r"(bar), "n"(T) : "memory"); }
 };
 
-template <uint32_t WARPS>
-__device__ __forceinline__ ListScan list_scan(const DevInstance &I, const uint32_t *summary, const uint32_t *mask, ListShared &L)
+template <uint32_t T, uint32_t CAP>
+struct ListChunk
 {
-	const unsigned full = 0xffffffffu;
-	const uint32_t lane = threadIdx.x & 31u, SW = I.summary_words;
-	// Four words at a time, so that their loads are in flight together.
-	for (uint32_t sw = threadIdx.x >> 5; sw < SW; sw += 4u * WARPS)
+	static constexpr uint32_t WARPS = T / 32u;
+	static_assert(LIST_WORDS == 4 && LIST_WORDS * WARPS <= 32, "two packed scans, one count per lane");
+	uint32_t words[LIST_WORDS];
+	uint32_t pos[LIST_WORDS]; // place of the thread's first index under each word
+	uint32_t total;
+
+	// Words [first, first + T * LIST_WORDS) of the `count` of the sub-tile.
+	__device__ __forceinline__ void load(const ShadeGroup<T> &G, const uint32_t *mask, uint32_t first, uint32_t count,
+	                                     ListShared<T, CAP> &L)
 	{
-		uint32_t words[4], mw[4];
+		const unsigned full = 0xffffffffu;
+		const uint32_t t = G.thread(), lane = t & 31u, warp = t >> 5;
 		#pragma unroll
-		for (int k = 0; k < 4; k++)
-			words[k] = sw + k * WARPS < SW ? __ldg(summary + sw + k * WARPS) : 0u;
+		for (uint32_t k = 0; k < LIST_WORDS; k++)
+			words[k] = first + k * T + t < count ? __ldg(mask + first + k * T + t) : 0u;
+		// Two words' counts (1024 at most in a warp) per scan.
+		const uint32_t c01 = uint32_t(__popc(words[0])) | (uint32_t(__popc(words[1])) << 16);
+		const uint32_t c23 = uint32_t(__popc(words[2])) | (uint32_t(__popc(words[3])) << 16);
+		const uint32_t x01 = warp_scan(c01, lane), x23 = warp_scan(c23, lane);
+		if (lane == 31u)
+		{
+			L.count[warp] = x01 & 0xffffu;
+			L.count[WARPS + warp] = x01 >> 16;
+			L.count[2u * WARPS + warp] = x23 & 0xffffu;
+			L.count[3u * WARPS + warp] = x23 >> 16;
+		}
+		G.sync();
+		const uint32_t v = lane < LIST_WORDS * WARPS ? L.count[lane] : 0u, x = warp_scan(v, lane);
+		total = __shfl_sync(full, x, 31);
+		const uint32_t e01 = x01 - c01, e23 = x23 - c23;
+		const uint32_t before[LIST_WORDS] = { e01 & 0xffffu, e01 >> 16, e23 & 0xffffu, e23 >> 16 };
 		#pragma unroll
-		for (int k = 0; k < 4; k++)
-			mw[k] = ((words[k] >> lane) & 1u) ? __ldg(mask + (sw + k * WARPS) * 32u + lane) : 0u;
-		#pragma unroll
-		for (int k = 0; k < 4; k++)
-			if (sw + k * WARPS < SW)
-			{
-				const uint32_t c = __reduce_add_sync(full, uint32_t(__popc(mw[k])));
-				if (lane == 0)
-					L.count[sw + k * WARPS] = c;
-			}
+		for (uint32_t k = 0; k < LIST_WORDS; k++)
+			pos[k] = __shfl_sync(full, x - v, int(k * WARPS + warp)) + before[k];
 	}
-	__syncthreads();
-	ListScan r;
-	const uint32_t v = lane < SW ? L.count[lane] : 0u, x = warp_scan(v, lane);
-	r.lo = x - v;
-	r.total = __shfl_sync(full, x, 31);
-	r.hi = 0;
-	if (SW > 32u)
+
+	// Indices [round, round + CAP) of the chunk.
+	__device__ __forceinline__ void write(const ShadeGroup<T> &G, uint32_t prim_lo, uint32_t first, uint32_t round,
+	                                      ListShared<T, CAP> &L) const
 	{
-		const uint32_t w = lane + 32u < SW ? L.count[lane + 32u] : 0u, y = warp_scan(w, lane);
-		r.hi = r.total + y - w;
-		r.total += __shfl_sync(full, y, 31);
+		#pragma unroll
+		for (uint32_t k = 0; k < LIST_WORDS; k++)
+		{
+			uint32_t p = pos[k] - round;
+			for (uint32_t m = words[k]; m; m &= m - 1u, p++)
+				if (p < CAP)
+					L.ids[p] = prim_lo + (first + k * T + G.thread()) * 32u + uint32_t(__ffs(m) - 1);
+		}
 	}
-	return r;
-}
+};
 
 // Walks the list: without AA1 through coverage masks (walk_batch); with AA1
 // every lane tests one primitive against the warp's rectangle (may_cover) and
 // the warp shades, in order, the primitives that can touch it, so that it sees
 // the same sequence of covering primitives as walking the whole list.
-template <int NS, bool SS, bool AA, bool MIP>
-__device__ __forceinline__ void walk_culled(const ShadeCtx &C, const DevInstance &I, const uint32_t *summary,
-                                            const uint32_t *mask, const ListScan &scan, ListShared &L, uint32_t t,
-                                            SampleState &S, uint32_t &covered)
+// `chunk` is the list's first chunk, loaded by the caller.
+template <int NS, bool SS, bool AA, bool MIP, uint32_t T, uint32_t CAP>
+__device__ __forceinline__ void walk_list(const ShadeCtx &C, const DevInstance &I, const ShadeGroup<T> &G, const uint32_t *mask,
+                                          ListChunk<T, CAP> &chunk, ListShared<T, CAP> &L, uint32_t t, SampleState &S,
+                                          uint32_t &covered)
 {
-	constexpr uint32_t WARPS = ShadeCta<NS>::WARPS;
-	__shared__ int4 s_rect[AA ? WARPS : 1];
-	__shared__ int2 s_smp[NS];
 	const PassParams &P = *C.P;
-	const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+	const uint32_t lane = threadIdx.x & 31u, warp = G.thread() >> 5;
 	const unsigned full = 0xffffffffu;
-	const uint32_t SW = I.summary_words;
 	WarpPlace W;
 	uint32_t my_bit = 0, even_rows = 0, even_pixels = 0;
 	if constexpr (!AA)
@@ -2691,10 +2677,10 @@ __device__ __forceinline__ void walk_culled(const ShadeCtx &C, const DevInstance
 		const int32_t px = S.hx >> C.dim, py = S.hy >> C.dim;
 		W.px0 = __shfl_sync(full, px, 0);
 		W.py0 = __shfl_sync(full, py, 0);
-		W.smp = s_smp;
+		W.smp = L.smp;
 		my_bit = B::bit(t % NS, uint32_t(px - W.px0), uint32_t(py - W.py0));
-		if (threadIdx.x < NS)
-			s_smp[threadIdx.x] = make_int2((S.hx - (px << C.dim)) << (3 - C.dim), (S.hy - (py << C.dim)) << (3 - C.dim));
+		if (G.thread() < NS)
+			L.smp[G.thread()] = make_int2((S.hx - (px << C.dim)) << (3 - C.dim), (S.hy - (py << C.dim)) << (3 - C.dim));
 		if (P.has_scanmsk)
 		{
 			even_rows = __reduce_or_sync(full, (S.hy & 1) ? 0u : 1u << my_bit);
@@ -2707,61 +2693,54 @@ __device__ __forceinline__ void walk_culled(const ShadeCtx &C, const DevInstance
 		const int4 r = make_int4(__reduce_min_sync(full, x0), __reduce_min_sync(full, y0),
 		                         __reduce_max_sync(full, S.hx), __reduce_max_sync(full, S.hy));
 		if (lane == 0)
-			s_rect[warp] = r;
+			L.rect[warp] = r;
 	}
-	const uint32_t total = scan.total;
-	for (uint32_t round = 0; round < total; round += LIST_CAP)
+	for (uint32_t first = 0;;)
 	{
-		for (uint32_t sw = warp; sw < SW; sw += WARPS)
+		const bool last_chunk = first + T * LIST_WORDS >= I.mask_words;
+		for (uint32_t round = 0; round < chunk.total || (last_chunk && round == 0); round += CAP)
 		{
-			const uint32_t off = __shfl_sync(full, sw < 32u ? scan.lo : scan.hi, int(sw & 31u)), count = L.count[sw];
-			if (!count || off + count <= round || off >= round + LIST_CAP)
-				continue;
-			const uint32_t words = __ldg(summary + sw);
-			const uint32_t mw = ((words >> lane) & 1u) ? __ldg(mask + sw * 32u + lane) : 0u;
-			const uint32_t pc = uint32_t(__popc(mw));
-			uint32_t pos = off + warp_scan(pc, lane) - pc;
-			const uint32_t prim_base = I.prim_lo + (sw * 32u + lane) * 32u;
-			for (uint32_t m = mw; m; m &= m - 1u, pos++)
-				if (pos >= round && pos < round + LIST_CAP)
-					L.ids[pos - round] = prim_base + uint32_t(__ffs(m) - 1);
-		}
-		__syncthreads();
-		const uint32_t n = min(total - round, LIST_CAP);
-		if constexpr (!AA)
-		{
+			if (round)
+				G.sync();
+			chunk.write(G, I.prim_lo, first, round, L);
+			G.sync();
+			const uint32_t n = min(chunk.total - round, CAP);
+			const bool last_round = last_chunk && round + CAP >= chunk.total;
+			if constexpr (!AA)
+			{
+				// The last batch, even an empty one, shades what is pending.
+				for (uint32_t kb = 0; kb < n || (last_round && kb == 0); kb += 32u)
+					walk_batch<NS, SS>(C, L.ids + kb, min(n - kb, 32u), W, my_bit, even_rows, even_pixels, last_round && kb + 32u >= n,
+					                   S, covered);
+			}
+			else
 			for (uint32_t kb = 0; kb < n; kb += 32u)
-				walk_batch<NS, SS>(C, L.ids + kb, min(n - kb, 32u), W, my_bit, even_rows, even_pixels, round + kb + 32u >= total, S,
-				                   covered);
-		}
-		else
-		for (uint32_t kb = 0; kb < n; kb += 32u)
-		{
-			const uint32_t k = kb + lane;
-			uint32_t pi = 0;
-			bool hit = false;
-			if (k < n)
 			{
-				pi = L.ids[k];
-				hit = may_cover<AA>(P.setup[pi], P.prims[pi].state, s_rect[warp], C.dim);
-			}
-			uint32_t bits = __ballot_sync(full, hit);
-			while (bits)
-			{
-				const int b = __ffs(bits) - 1;
-				bits &= bits - 1u;
-				process_primitive<SS, AA, MIP>(C, __shfl_sync(full, pi, b), S, covered);
+				const uint32_t k = kb + lane;
+				uint32_t pi = 0;
+				bool hit = false;
+				if (k < n)
+				{
+					pi = L.ids[k];
+					hit = may_cover(P.setup[pi], P.prims[pi].state, L.rect[warp], C.dim);
+				}
+				uint32_t bits = __ballot_sync(full, hit);
+				while (bits)
+				{
+					const int b = __ffs(bits) - 1;
+					bits &= bits - 1u;
+					process_primitive<SS, MIP>(C, __shfl_sync(full, pi, b), S, covered);
+				}
 			}
 		}
-		if (round + LIST_CAP < total)
-			__syncthreads();
+		if (last_chunk)
+			break;
+		first += T * LIST_WORDS;
+		G.sync();
+		chunk.load(G, mask, first, I.mask_words, L);
 	}
 }
 
-// One CTA per 8x8-pixel sub-tile, NS samples per pixel, one thread per sample.
-// Each warp walks the sub-tile's primitive bitmask on its own (no shared
-// memory, no barriers).  SS selects the super-sampled path; sub-tiles whose
-// coarse tile selects the other path exit immediately.
 // Coarse-tile state of sub-tile `sub`: 0 = empty, 1 = single-sampled,
 // 2 = super-sampled (binning.comp:272-311 decision).
 __device__ __forceinline__ uint32_t subtile_mode(const PassParams &P, const DevInstance &I, const uint32_t *tile_flags,
@@ -2779,27 +2758,22 @@ __device__ __forceinline__ uint32_t subtile_mode(const PassParams &P, const DevI
 	return (I.rate_y_log2 != 0 && req) ? 2u : 1u;
 }
 
-// One sub-tile's pixel samples; `t` is the thread's index among the 64 * NS
-// threads that cover the sub-tile.  CULL: the whole CTA runs the sub-tile and
-// walks its primitive list together (walk_culled); otherwise each warp walks
-// the sub-tile's primitive bitmask on its own and needs no barrier.
-template <int NS, bool SS, bool AA, bool MIP = false, bool CULL = false>
-__device__ __forceinline__ void shade_subtile(const PassParams &P, const DevInstance &I, const uint32_t *sub_masks,
-                                              const uint32_t *sub_summary, uint32_t sub, uint32_t t, ListShared *list = nullptr)
+// One sub-tile's pixel samples, NS per pixel, one thread per sample: the T
+// threads of the group have samples t (of 64 * NS) of it, as many as there are or
+// a part of them.  SS selects the super-sampled path.
+template <int NS, bool SS, bool AA, bool MIP, uint32_t T, uint32_t CAP>
+__device__ __forceinline__ void shade_subtile(const PassParams &P, const DevInstance &I, const ShadeGroup<T> &G,
+                                              const uint32_t *sub_masks, uint32_t sub, uint32_t t, ListShared<T, CAP> &list)
 {
 	const uint32_t gx = sub % I.sub_w, gy = sub / I.sub_w;
-	const uint32_t *summary = sub_summary + size_t(sub) * I.summary_words;
 	const uint32_t *mask = sub_masks + size_t(sub) * I.mask_words;
 
-	// The list first: most sub-tiles of a pass of small primitives have none,
+	// The list first: many sub-tiles of a pass of small primitives have none,
 	// and the samples' loads overlap its expansion.
-	ListScan scan = {};
-	if constexpr (CULL)
-	{
-		scan = list_scan<ShadeCta<NS>::WARPS>(I, summary, mask, *list);
-		if (!scan.total)
-			return;
-	}
+	ListChunk<T, CAP> chunk;
+	chunk.load(G, mask, 0, I.mask_words, list);
+	if (!chunk.total && I.mask_words <= T * LIST_WORDS)
+		return;
 
 	ShadeCtx C;
 	C.P = &P;
@@ -2888,40 +2862,11 @@ __device__ __forceinline__ void shade_subtile(const PassParams &P, const DevInst
 	else
 		S.depth = 0;
 
-	// Walk the primitive list in ascending order: summary word -> mask words -> bits.
 	uint32_t covered = 0;
-	if constexpr (CULL)
-		walk_culled<NS, SS, AA, MIP>(C, I, summary, mask, scan, *list, t, S, covered);
-	else
-	for (uint32_t sbase = 0; sbase < I.summary_words; sbase += 32u)
-	{
-		uint32_t sv = (sbase + lane < I.summary_words) ? __ldg(summary + sbase + lane) : 0u;
-		uint32_t nz_lanes = __ballot_sync(0xffffffffu, sv != 0u);
-		while (nz_lanes)
-		{
-			int l = __ffs(nz_lanes) - 1;
-			nz_lanes &= nz_lanes - 1u;
-			uint32_t words = __shfl_sync(0xffffffffu, sv, l);
-			uint32_t word_base = (sbase + uint32_t(l)) * 32u;
-			uint32_t mw = ((words >> lane) & 1u) ? __ldg(mask + word_base + lane) : 0u;
-			while (words)
-			{
-				int j = __ffs(words) - 1;
-				words &= words - 1u;
-				uint32_t m = __shfl_sync(0xffffffffu, mw, j);
-				uint32_t prim_base = I.prim_lo + (word_base + uint32_t(j)) * 32u;
-				while (m)
-				{
-					int b = __ffs(m) - 1;
-					m &= m - 1u;
-					process_primitive<SS, AA, MIP>(C, prim_base + uint32_t(b), S, covered);
-				}
-			}
-		}
-	}
+	walk_list<NS, SS, AA, MIP, T, CAP>(C, I, G, mask, chunk, list, t, S, covered);
 
 	// walk_batch leaves nothing pending.
-	if ((AA || !CULL) && S.pending.coverage > 0)
+	if (AA && S.pending.coverage > 0)
 		shade_resolve<MIP, AA>(C, S, S.pending_prim, S.pending);
 
 	// Covered-sample counter: one atomic per warp.
@@ -3035,33 +2980,41 @@ __device__ __forceinline__ void shade_subtile(const PassParams &P, const DevInst
 	}
 }
 
+// Indices held in shared memory at a time.
+constexpr uint32_t SHADE_LIST_CAP = 2048u, BATCH_LIST_CAP = 512u;
+
+// Sub-tiles whose coarse tile selects the other path exit immediately.
 template <int NS, bool SS, bool AA, bool MIP>
 __global__ void __launch_bounds__(ShadeCta<NS>::THREADS, PGS_SHADE_MIN_BLOCKS(NS, AA || MIP)) shade_kernel(PassParams P, DevInstance I, const uint32_t *sub_masks,
-                                                        const uint32_t *sub_summary, const uint32_t *tile_flags)
+                                                        const uint32_t *tile_flags)
 {
-	constexpr uint32_t PARTS = ShadeCta<NS>::PARTS;
-	__shared__ ListShared list;
+	constexpr uint32_t T = ShadeCta<NS>::THREADS, PARTS = ShadeCta<NS>::PARTS;
+	__shared__ ListShared<T, SHADE_LIST_CAP> list;
 	const uint32_t sub = blockIdx.x / PARTS, part = blockIdx.x % PARTS;
 	if (sub >= I.sub_w * I.sub_h)
 		return;
 	if (subtile_mode(P, I, tile_flags, sub) != (SS ? 2u : 1u))
 		return;
-	shade_subtile<NS, SS, AA, MIP, true>(P, I, sub_masks, sub_summary, sub, part * ShadeCta<NS>::THREADS + threadIdx.x, &list);
+	shade_subtile<NS, SS, AA, MIP, T, SHADE_LIST_CAP>(P, I, ShadeGroup<T>{ 0u }, sub_masks, sub, part * T + threadIdx.x, list);
 }
 
 // ---------------------------------------------------------------------------
 // Batched shading: one launch shades the current instance segment of many
-// independent command streams.  Each item is one (stream, pass, segment)
-// with its own VRAM, records and bins; its work is cut into warp units
-// (sub-tile, warp) -- 2 * 2^ns_log2 units per sub-tile, of which a
-// single-sampled tile uses the first two -- that persistent warps take from a
-// global counter, so streams of very different sizes share the GPU without
-// a tail per stream.
+// independent command streams.  Each item is one (stream, pass, segment) with
+// its own VRAM, records and bins; its samples, sub-tile after sub-tile, are cut
+// into units of BLOCK that persistent CTAs take from a global counter, so
+// streams of very different sizes share the GPU without a tail per stream.  In a
+// unit the threads of each sub-tile form a group that expands and walks the
+// sub-tile's list as a CTA of shade_kernel does (of a single-sampled sub-tile the
+// first 64 threads do).
+// Bound: issue of the shading itself, as in shade_kernel.  The five smallest of
+// twelve mixed streams took 285 us in units of one warp, each of which walked its
+// sub-tile's whole list on its own, and take 276 us.
 struct ShadeItem
 {
 	PassParams P;
 	DevInstance I;
-	const uint32_t *masks, *summary, *flags;
+	const uint32_t *masks, *flags;
 	uint32_t ns_log2, aa;
 	uint32_t unit_base, units;
 };
@@ -3071,30 +3024,42 @@ constexpr uint32_t BATCH_MAX_NS_LOG2 = 2;
 
 // Separate functions per variant keep each variant's register allocation
 // its own inside the batched kernel.
-template <int NS, bool SS, bool AA>
-__device__ __noinline__ void shade_subtile_call(const PassParams &P, const DevInstance &I, const uint32_t *sub_masks,
-                                                const uint32_t *sub_summary, uint32_t sub, uint32_t t)
+template <int NS, bool SS, bool AA, uint32_t T>
+__device__ __noinline__ void shade_subtile_call(const PassParams &P, const DevInstance &I, const uint32_t *sub_masks, uint32_t sub,
+                                                uint32_t t, uint32_t bar, ListShared<T, BATCH_LIST_CAP> &list)
 {
-	shade_subtile<NS, SS, AA>(P, I, sub_masks, sub_summary, sub, t);
+	shade_subtile<NS, SS, AA, false, T, BATCH_LIST_CAP>(P, I, ShadeGroup<T>{ bar }, sub_masks, sub, t, list);
 }
 
 template <int BLOCK>
 __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) batch_shade_kernel(const ShadeItem *items, uint32_t n_items,
                                                                          uint32_t total_units, uint32_t *counter)
 {
-	constexpr int WARPS = BLOCK / 32;
-	__shared__ PassParams sP[WARPS];
-	__shared__ DevInstance sI[WARPS];
-	const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
-	uint32_t loaded = 0xffffffffu;
-	for (;;)
+	constexpr uint32_t T4 = BLOCK < 256 ? BLOCK : 256, T2 = 128, T1 = 64;
+	// One list per 64 threads; a group of several uses the first of its own.
+	struct Slot
 	{
-		uint32_t unit = 0;
-		if (lane == 0)
-			unit = atomicAdd(counter, 1u);
-		unit = __shfl_sync(0xffffffffu, unit, 0);
+		ListShared<T1, BATCH_LIST_CAP> list;
+	};
+	static_assert(sizeof(ListShared<T4, BATCH_LIST_CAP>) <= (T4 / T1) * sizeof(Slot) &&
+	                  sizeof(ListShared<T2, BATCH_LIST_CAP>) <= (T2 / T1) * sizeof(Slot),
+	              "a group's list fits its slots");
+	__shared__ PassParams P;
+	__shared__ DevInstance I;
+	__shared__ Slot slots[BLOCK / T1];
+	__shared__ uint32_t s_unit[2];
+	if (threadIdx.x == 0)
+		s_unit[0] = atomicAdd(counter, 1u);
+	__syncthreads();
+	uint32_t loaded = 0xffffffffu;
+	for (uint32_t step = 0;; step++)
+	{
+		const uint32_t unit = s_unit[step & 1u];
 		if (unit >= total_units)
 			break;
+		// The next unit's number is on its way while this one is shaded.
+		if (threadIdx.x == 0)
+			s_unit[(step + 1u) & 1u] = atomicAdd(counter, 1u);
 		uint32_t lo = 0, hi = n_items - 1;
 		while (lo < hi)
 		{
@@ -3107,47 +3072,47 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) batch_shade_kernel(const 
 		const ShadeItem &it = items[lo];
 		if (lo != loaded)
 		{
-			// Item parameters into this warp's shared slot.
-			__syncwarp();
-			const uint32_t *srcP = reinterpret_cast<const uint32_t *>(&it.P);
-			uint32_t *dstP = reinterpret_cast<uint32_t *>(&sP[warp]);
-			for (uint32_t k = lane; k < sizeof(PassParams) / 4; k += 32u)
-				dstP[k] = srcP[k];
-			const uint32_t *srcI = reinterpret_cast<const uint32_t *>(&it.I);
-			uint32_t *dstI = reinterpret_cast<uint32_t *>(&sI[warp]);
-			for (uint32_t k = lane; k < sizeof(DevInstance) / 4; k += 32u)
-				dstI[k] = srcI[k];
-			__syncwarp();
+			// Item parameters into shared memory (all are done with the last item's).
+			const uint32_t *srcP = reinterpret_cast<const uint32_t *>(&it.P), *srcI = reinterpret_cast<const uint32_t *>(&it.I);
+			for (uint32_t k = threadIdx.x; k < sizeof(PassParams) / 4; k += BLOCK)
+				reinterpret_cast<uint32_t *>(&P)[k] = srcP[k];
+			for (uint32_t k = threadIdx.x; k < sizeof(DevInstance) / 4; k += BLOCK)
+				reinterpret_cast<uint32_t *>(&I)[k] = srcI[k];
 			loaded = lo;
+			__syncthreads();
 		}
-		const PassParams &P = sP[warp];
-		const DevInstance &I = sI[warp];
-		const uint32_t local = unit - it.unit_base;
-		const uint32_t per_sub = 2u << it.ns_log2;
-		const uint32_t sub = local / per_sub, w = local % per_sub;
-		const uint32_t mode = subtile_mode(P, I, it.flags, sub);
-		if (mode == 0)
-			continue;
+		const uint32_t sample = (unit - it.unit_base) * BLOCK + threadIdx.x;
+		const uint32_t sub = sample >> (6u + it.ns_log2), t = sample & ((64u << it.ns_log2) - 1u);
+		const uint32_t mode = sub < I.sub_w * I.sub_h ? subtile_mode(P, I, it.flags, sub) : 0u;
 		const uint32_t ns_log2 = mode == 2 ? it.ns_log2 : 0u;
-		if (w >= (2u << ns_log2))
-			continue;
-		const uint32_t t = w * 32u + lane;
-		const bool aa = it.aa != 0;
-		switch (ns_log2)
+		// A group's barrier and list are those of its first 64 threads.
+		if (mode && t < (64u << ns_log2))
 		{
-		case 0:
-			if (aa) shade_subtile_call<1, false, true>(P, I, it.masks, it.summary, sub, t);
-			else shade_subtile_call<1, false, false>(P, I, it.masks, it.summary, sub, t);
-			break;
-		case 1:
-			if (aa) shade_subtile_call<2, true, true>(P, I, it.masks, it.summary, sub, t);
-			else shade_subtile_call<2, true, false>(P, I, it.masks, it.summary, sub, t);
-			break;
-		default:
-			if (aa) shade_subtile_call<4, true, true>(P, I, it.masks, it.summary, sub, t);
-			else shade_subtile_call<4, true, false>(P, I, it.masks, it.summary, sub, t);
-			break;
+			const bool aa = it.aa != 0;
+			const uint32_t s4 = threadIdx.x / T4 * (T4 / T1), s2 = threadIdx.x / T2 * (T2 / T1), s1 = threadIdx.x / T1;
+			switch (ns_log2)
+			{
+			case 0:
+				if (aa) shade_subtile_call<1, false, true, T1>(P, I, it.masks, sub, t, 1u + s1, slots[s1].list);
+				else shade_subtile_call<1, false, false, T1>(P, I, it.masks, sub, t, 1u + s1, slots[s1].list);
+				break;
+			case 1:
+			{
+				auto &list = reinterpret_cast<ListShared<T2, BATCH_LIST_CAP> &>(slots[s2]);
+				if (aa) shade_subtile_call<2, true, true, T2>(P, I, it.masks, sub, t, 1u + s2, list);
+				else shade_subtile_call<2, true, false, T2>(P, I, it.masks, sub, t, 1u + s2, list);
+				break;
+			}
+			default:
+			{
+				auto &list = reinterpret_cast<ListShared<T4, BATCH_LIST_CAP> &>(slots[s4]);
+				if (aa) shade_subtile_call<4, true, true, T4>(P, I, it.masks, sub, t, 1u + s4, list);
+				else shade_subtile_call<4, true, false, T4>(P, I, it.masks, sub, t, 1u + s4, list);
+				break;
+			}
+			}
 		}
+		__syncthreads();
 	}
 }
 

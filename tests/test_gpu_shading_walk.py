@@ -9,6 +9,7 @@ import pytest
 
 import gsgen
 import pgs
+import pgs_oracle
 from test_gpu_parity import assert_same, run_both
 
 pytestmark = pytest.mark.gpu
@@ -133,3 +134,46 @@ def test_blend_alpha_and_wrap_states(fpsm, ss):
                  [gsgen.D_UV if fst else gsgen.D_ST, gsgen.D_RGBAQ, gsgen.D_XYZ2], q.reshape(-1, 2))
         total += n
     assert_same(*run_both(frame(s, ss, True, total)))
+
+
+@pytest.mark.parametrize("cta_threads", [128, 256, 512])
+def test_batched_rounds(cta_threads):
+    """Streams of every rate share the rounds: single-sampled tiles inside a
+    super-sampled stream, a sub-tile's list past the batched kernel's 512 and the
+    mask words past one chunk of 64 threads (8192 primitives)."""
+    rng = np.random.default_rng(cta_threads)
+    frames = []
+    for ss, ordered, n in ((1, True, 8300), (2, True, 700), (4, False, 600), (4, True, 40)):
+        s = gsgen.GifStream()
+        setup(s, gsgen.PSMCT32, gsgen.PSMZ24)
+        triangles(s, rng, n, 8, 8, 8, rng.integers(0, 1 << 24, size=(n, 3)))
+        triangles(s, rng, 9, 0, 0, 96, rng.integers(0, 1 << 24, size=(9, 3)), abe=1)
+        # Flat sprites on pixel boundaries, away from the rest: tiles that need one sample.
+        x = np.array([[100, 126]] * 3) * 16
+        q = np.zeros((6, 2, 2), dtype=np.uint64)
+        q[:, 0] = gsgen.q_rgbaq(rng.integers(0, 256, size=(6, 4), dtype=np.int64))
+        q[:, 1] = gsgen.q_xyz2(x.reshape(-1), x.reshape(-1) - 40 * 16, np.full(6, 77))
+        s.packed(gsgen.prim_reg(gsgen.PRIM_SPRITE), [gsgen.D_RGBAQ, gsgen.D_XYZ2], q.reshape(-1, 2))
+        frames.append(frame(s, ss, ordered, n + 12))
+    backends, batch = [], pgs.Batch(0)
+    try:
+        for f in frames:
+            be = pgs.CudaBackend(0, max_samples_log2=2)
+            backends.append(be)
+            gs = pgs.GSInterface(be, super_sampling=f.super_sampling, ordered=f.ordered)
+            be.begin_record()
+            gs.gif_transfer(0, f.data)
+            gs.flush()
+            be.end_record()
+            gs.close()
+            batch.add(be)
+        batch.set_tuning(cta_threads, 1024 // cta_threads, True, 0)
+        batch.replay(1)
+        batch.synchronize()
+        for be, f in zip(backends, frames):
+            ref = pgs_oracle.render(f, planes=True)
+            assert_same(ref, np.stack([be.read_plane(p) for p in range(ref.shape[0])]))
+    finally:
+        batch.close()
+        for be in backends:
+            be.close()
