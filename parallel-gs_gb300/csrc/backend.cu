@@ -246,6 +246,8 @@ static TexAxis sampler_axis(bool perspective, bool clamp, uint32_t mode, uint32_
 	return a;
 }
 
+constexpr size_t CLUT_BYTES = size_t(PGS_CLUT_INSTANCES) * PGS_CLUT_SIZE_BYTES;
+
 struct CudaBackend
 {
 	int device = 0;
@@ -315,8 +317,7 @@ struct CudaBackend
 	std::vector<Op> ops;
 	std::vector<uint64_t> batch_blocks;
 	std::vector<uint32_t> scratch_blocks;
-	uint8_t *d_reset_vram = nullptr;
-	uint16_t *d_reset_clut = nullptr;
+	uint8_t *d_reset = nullptr; // CLUT ring and VRAM as the recording began
 	uint32_t reset_planes = 0;
 	cudaGraphExec_t graph_exec = nullptr;
 	uint32_t launches_per_replay = 0;
@@ -436,10 +437,10 @@ struct CudaBackend
 		CUDA_TRY(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
 		uint32_t ms = opt ? std::min<uint32_t>(opt->max_samples_log2, 4) : 4;
 		max_planes = ms ? 2u + (1u << ms) : 1u;
-		CUDA_TRY(cudaMalloc(&d_vram, size_t(max_planes) * VRAM_SIZE));
-		CUDA_TRY(cudaMemset(d_vram, 0, size_t(max_planes) * VRAM_SIZE));
-		CUDA_TRY(cudaMalloc(&d_clut, size_t(PGS_CLUT_INSTANCES) * PGS_CLUT_SIZE_BYTES));
-		CUDA_TRY(cudaMemset(d_clut, 0, size_t(PGS_CLUT_INSTANCES) * PGS_CLUT_SIZE_BYTES));
+		// The CLUT ring, then VRAM: a replay restores both with one copy.
+		CUDA_TRY(cudaMalloc(&d_clut, CLUT_BYTES + size_t(max_planes) * VRAM_SIZE));
+		CUDA_TRY(cudaMemset(d_clut, 0, CLUT_BYTES + size_t(max_planes) * VRAM_SIZE));
+		d_vram = reinterpret_cast<uint8_t *>(d_clut) + CLUT_BYTES;
 		CUDA_TRY(cudaMalloc(&d_snapshot, VRAM_SIZE));
 		CUDA_TRY(cudaMalloc(&d_error, sizeof(uint32_t)));
 		CUDA_TRY(cudaMemset(d_error, 0, sizeof(uint32_t)));
@@ -510,7 +511,6 @@ struct CudaBackend
 			cudaStreamSynchronize(stream);
 		if (graph_exec)
 			cudaGraphExecDestroy(graph_exec);
-		cudaFree(d_vram);
 		cudaFree(d_clut);
 		cudaFree(d_snapshot);
 		for (auto &p : d_tex_snap)
@@ -537,8 +537,7 @@ struct CudaBackend
 		                      &vs_fields[2], &vs_fields[3] })
 			cudaFree(im->ptr);
 		cudaFree(d_arena);
-		cudaFree(d_reset_vram);
-		cudaFree(d_reset_clut);
+		cudaFree(d_reset);
 		cudaFreeHost(h_arena);
 		for (int i = 0; i < MAX_STAGES; i++)
 		{
@@ -1537,6 +1536,7 @@ struct CudaBackend
 		// Setup and the single-sample heuristic rewrite primitive words in
 		// place: a recorded pass works on a copy so that its records stay as
 		// recorded for the next replay; a pass run once works on its records.
+		P.prims_in = reinterpret_cast<const pgs_primitive_attribute *>(d_arena + p.prim_off);
 		P.prims = live_op ? reinterpret_cast<pgs_primitive_attribute *>(d_arena + p.prim_off) : d_prims_work;
 		P.setup = d_setup;
 		P.tattr = d_tattr;
@@ -1569,9 +1569,6 @@ struct CudaBackend
 			P.setup_rate_x_log2 = std::max(P.setup_rate_x_log2, p.instances[i].sampling_rate_x_log2);
 			P.setup_rate_y_log2 = std::max(P.setup_rate_y_log2, p.instances[i].sampling_rate_y_log2);
 		}
-		if (!live_op)
-			CUDA_TRY(cudaMemcpyAsync(d_prims_work, d_arena + p.prim_off, size_t(p.num_prims) * sizeof(pgs_primitive_attribute),
-			                         cudaMemcpyDeviceToDevice, stream));
 		{
 			StageScope ts(this, PGS_TIMESTAMP_TRIANGLE_SETUP);
 			if (H.instance_mask)
@@ -2086,15 +2083,10 @@ struct CudaBackend
 		op_blocks_state.clear();
 		arena_used = 0;
 		size_t vbytes = size_t(num_planes) * VRAM_SIZE;
-		cudaFree(d_reset_vram);
-		cudaFree(d_reset_clut);
-		d_reset_vram = nullptr;
-		d_reset_clut = nullptr;
-		CUDA_TRY(cudaMalloc(&d_reset_vram, vbytes));
-		CUDA_TRY(cudaMalloc(&d_reset_clut, size_t(PGS_CLUT_INSTANCES) * PGS_CLUT_SIZE_BYTES));
-		CUDA_TRY(cudaMemcpyAsync(d_reset_vram, d_vram, vbytes, cudaMemcpyDeviceToDevice, stream));
-		CUDA_TRY(cudaMemcpyAsync(d_reset_clut, d_clut, size_t(PGS_CLUT_INSTANCES) * PGS_CLUT_SIZE_BYTES,
-		                         cudaMemcpyDeviceToDevice, stream));
+		cudaFree(d_reset);
+		d_reset = nullptr;
+		CUDA_TRY(cudaMalloc(&d_reset, CLUT_BYTES + vbytes));
+		CUDA_TRY(cudaMemcpyAsync(d_reset, d_clut, CLUT_BYTES + vbytes, cudaMemcpyDeviceToDevice, stream));
 		reset_planes = num_planes;
 		recording = true;
 		return PGS_OK;
@@ -2107,15 +2099,22 @@ struct CudaBackend
 		return PGS_OK;
 	}
 
+	// The CLUT ring and VRAM as the recording began.
+	int restore()
+	{
+		CUDA_TRY(cudaMemcpyAsync(d_clut, d_reset, CLUT_BYTES + size_t(reset_planes) * VRAM_SIZE, cudaMemcpyDeviceToDevice, stream));
+		return PGS_OK;
+	}
+
 	int replay_once(bool reset)
 	{
 		launch_counter = 0;
 		shade_started = false;
-		if (reset && d_reset_vram)
+		if (reset && d_reset)
 		{
-			CUDA_TRY(cudaMemcpyAsync(d_vram, d_reset_vram, size_t(reset_planes) * VRAM_SIZE, cudaMemcpyDeviceToDevice, stream));
-			CUDA_TRY(cudaMemcpyAsync(d_clut, d_reset_clut, size_t(PGS_CLUT_INSTANCES) * PGS_CLUT_SIZE_BYTES,
-			                         cudaMemcpyDeviceToDevice, stream));
+			int r = restore();
+			if (r)
+				return r;
 		}
 		for (size_t i = 0; i < ops.size();)
 		{
@@ -2237,7 +2236,7 @@ struct BatchEngine
 
 	int add(CudaBackend *b)
 	{
-		if (b->device != device || b->ops.empty() || !b->d_reset_vram)
+		if (b->device != device || b->ops.empty() || !b->d_reset)
 			return PGS_ERROR_INVALID_ARGUMENT;
 		cudaEvent_t e;
 		CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
@@ -2329,12 +2328,8 @@ struct BatchEngine
 			return r;
 		if (reset)
 			for (CudaBackend *b : streams)
-			{
-				CUDA_TRY(cudaMemcpyAsync(b->d_vram, b->d_reset_vram, size_t(b->reset_planes) * VRAM_SIZE,
-				                         cudaMemcpyDeviceToDevice, b->stream));
-				CUDA_TRY(cudaMemcpyAsync(b->d_clut, b->d_reset_clut, size_t(PGS_CLUT_INSTANCES) * PGS_CLUT_SIZE_BYTES,
-				                         cudaMemcpyDeviceToDevice, b->stream));
-			}
+				if ((r = b->restore()))
+					return r;
 		// Solo streams: the whole frame on the stream's own CUDA stream.
 		for (size_t s = 0; s < streams.size(); s++)
 		{

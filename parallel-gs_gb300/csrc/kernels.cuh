@@ -163,6 +163,9 @@ struct PassParams
 	uint32_t num_snaps;
 	const pgs_vertex_position *pos;
 	const pgs_vertex_attribute *attr;
+	// Primitive words: setup reads them from prims_in and writes prims, which the
+	// kernels after it use (the same array where a pass is run once).
+	const pgs_primitive_attribute *prims_in;
 	pgs_primitive_attribute *prims;
 	const pgs_state_vector *states;
 	const pgs_texture_desc *textures;
@@ -335,7 +338,7 @@ __global__ void __launch_bounds__(128) setup_kernel(PassParams P)
 	if (index >= P.num_prims)
 		return;
 
-	pgs_primitive_attribute pa = P.prims[index];
+	pgs_primitive_attribute pa = P.prims_in[index];
 	PrimSetup out;
 	TransformedAttr ta;
 	const int sry = int(P.setup_rate_y_log2);
@@ -416,7 +419,8 @@ __global__ void __launch_bounds__(128) setup_kernel(PassParams P)
 		out.bb[0] = 0; out.bb[1] = 0; out.bb[2] = -1; out.bb[3] = -1;
 		reinterpret_cast<int4 *>(&P.setup[index])[3] = make_int4(0, 0, -1, -1);
 		if (sry != 0)
-			P.prims[index].state = st | (1u << STATE_BIT_SNAP_ATTRIBUTE);
+			pa.state = st | (1u << STATE_BIT_SNAP_ATTRIBUTE);
+		P.prims[index] = pa;
 		return;
 	}
 
@@ -742,8 +746,9 @@ __global__ void __launch_bounds__(128) setup_kernel(PassParams P)
 
 	P.setup[index] = out;
 	P.tattr[index] = ta;
-	P.prims[index].state = new_state;
-	P.prims[index].tex = tex;
+	pa.state = new_state;
+	pa.tex = tex;
+	P.prims[index] = pa;
 }
 
 // ---------------------------------------------------------------------------
