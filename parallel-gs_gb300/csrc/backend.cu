@@ -1092,10 +1092,10 @@ struct CudaBackend
 		{
 			switch (ns_log2)
 			{
-			case 1: shade_kernel<2, true, AA, MIP><<<grid * ShadeCta<2>::PARTS, ShadeCta<2>::THREADS, 0, stream>>>(P, I, masks, d_flags); break;
-			case 2: shade_kernel<4, true, AA, MIP><<<grid * ShadeCta<4>::PARTS, ShadeCta<4>::THREADS, 0, stream>>>(P, I, masks, d_flags); break;
-			case 3: shade_kernel<8, true, AA, MIP><<<grid * ShadeCta<8>::PARTS, ShadeCta<8>::THREADS, 0, stream>>>(P, I, masks, d_flags); break;
-			default: shade_kernel<16, true, AA, MIP><<<grid * ShadeCta<16>::PARTS, ShadeCta<16>::THREADS, 0, stream>>>(P, I, masks, d_flags); break;
+			case 1: shade_kernel<2, true, AA, MIP><<<grid, ShadeCta<2>::THREADS, 0, stream>>>(P, I, masks, d_flags); break;
+			case 2: shade_kernel<4, true, AA, MIP><<<grid, ShadeCta<4>::THREADS, 0, stream>>>(P, I, masks, d_flags); break;
+			case 3: shade_kernel<8, true, AA, MIP><<<grid, ShadeCta<8>::THREADS, 0, stream>>>(P, I, masks, d_flags); break;
+			default: shade_kernel<16, true, AA, MIP><<<grid, ShadeCta<16>::THREADS, 0, stream>>>(P, I, masks, d_flags); break;
 			}
 			launch_counter++;
 		}

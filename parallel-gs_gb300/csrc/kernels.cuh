@@ -213,24 +213,19 @@ constexpr uint32_t ERROR_FLAG_TILE_OVERFLOW = 1u << 0;
 __constant__ uint8_t c_rcp_tab[256];
 
 // Largest shading CTA, as the sampling rate it holds a whole sub-tile of, and
-// occupancy targets of the shading kernels in 256-thread units per SM: 4 means
-// at most 64 registers per thread.  Up to 4x the walk is bound by issue and
-// spills cost more than warps bring (textured 4x frame, 52,000 primitives: 4 CTAs
-// 618 us, 5 631 us, 6 642 us).  The plain variants (no AA1, no mipmaps) at 8x
-// and 16x wait on loads with few primitives per sub-tile (feedback frame, 100,000
-// primitives in ten passes, at 16x: 4 CTAs 4.02 ms, 5 3.79 ms, 6 3.66 ms).  CTA
-// size on the same frame at 16x: 128 threads 3.91 ms, 256 3.79 ms, 512 4.22 ms.
+// occupancy target of the shading kernels in 256-thread units per SM: 4 means at
+// most 64 registers per thread.  Textured 4x frame of 52,000 primitives: 4 CTAs
+// 618 us, 5 631 us, 6 642 us; 128 threads 596 us where 256 take 560.  Plain 1x
+// frame at 10, 12, 16, 20, 24 CTAs of 64 threads: 55, 48.5, 47, 50, 64 us.
+// Feedback frame of 100,000 primitives at 16x: 4 CTAs 2.74 ms (alone 3.28), 5
+// 2.74 (3.33), 6 2.81 (3.48).
 #ifndef PGS_SHADE_CTA_NS
 #define PGS_SHADE_CTA_NS 4
 #endif
 #ifndef PGS_SHADE_OCC
 #define PGS_SHADE_OCC 4
 #endif
-#ifndef PGS_SHADE_OCC_HIGH_RATE
-#define PGS_SHADE_OCC_HIGH_RATE 6
-#endif
-#define PGS_SHADE_MIN_BLOCKS(NS, LARGE) \
-	(((NS) >= 8 && !(LARGE) ? PGS_SHADE_OCC_HIGH_RATE : PGS_SHADE_OCC) * 4 / ((NS) < PGS_SHADE_CTA_NS ? (NS) : PGS_SHADE_CTA_NS))
+#define PGS_SHADE_MIN_BLOCKS(NS) (PGS_SHADE_OCC * 4 / ((NS) < PGS_SHADE_CTA_NS ? (NS) : PGS_SHADE_CTA_NS))
 
 // ---------------------------------------------------------------------------
 // Scalar helpers.
@@ -2603,16 +2598,17 @@ __device__ __forceinline__ void walk_batch(const ShadeCtx &C, const uint32_t *id
 	}
 }
 
-// Threads of a shading CTA: the 64 * NS samples of a sub-tile, in CTAs of 256 at
-// most.  The CTAs of a sub-tile expand its list each for themselves, which is
-// cheap next to what whole-sub-tile CTAs of 512 and 1024 threads cost at 8x and
-// 16x, two and one of them per SM, waiting for each other at every barrier:
-// feedback frame of 100,000 primitives, 8x 2.48 -> 2.07 ms, 16x 5.07 -> 3.66 ms.
+// Threads of a shading CTA: the 64 * NS samples of a sub-tile, 256 at most at a
+// time; a CTA runs a sub-tile's parts one after the other on one expanded list.
+// Whole sub-tiles in CTAs of 512 and 1024 threads at 8x and 16x leave two and one
+// of them per SM, waiting for each other at every barrier; a CTA per part expands
+// the list again and starts more CTAs (feedback frame of 100,000 primitives at 8x
+// 2.48 ms whole, 1.93 a CTA per part, 1.72 so; at 16x 5.07, 3.51, 2.74).
 template <int NS>
 struct ShadeCta
 {
 	static constexpr uint32_t THREADS = NS < PGS_SHADE_CTA_NS ? 64u * NS : 64u * PGS_SHADE_CTA_NS;
-	static constexpr uint32_t PARTS = 64u * NS / THREADS; // CTAs per sub-tile
+	static constexpr uint32_t PARTS = 64u * NS / THREADS;
 	static constexpr uint32_t WARPS = THREADS / 32u;
 };
 
@@ -2707,11 +2703,12 @@ struct ListChunk
 // every lane tests one primitive against the warp's rectangle (may_cover) and
 // the warp shades, in order, the primitives that can touch it, so that it sees
 // the same sequence of covering primitives as walking the whole list.
-// `chunk` is the list's first chunk, loaded by the caller.
-template <int NS, bool SS, bool AA, bool MIP, uint32_t T, uint32_t CAP>
+// `chunk` is the list's first chunk, loaded by the caller; with `written`, it is
+// the whole list and lies in L already.  RELOAD: the caller kept only its length.
+template <int NS, bool SS, bool AA, bool MIP, bool RELOAD, uint32_t T, uint32_t CAP>
 __device__ __forceinline__ void walk_list(const ShadeCtx &C, const DevInstance &I, const ShadeGroup<T> &G, const uint32_t *mask,
-                                          ListChunk<T, CAP> &chunk, ListShared<T, CAP> &L, uint32_t t, SampleState &S,
-                                          uint32_t &covered)
+                                          ListChunk<T, CAP> &chunk, bool written, ListShared<T, CAP> &L, uint32_t t,
+                                          SampleState &S, uint32_t &covered)
 {
 	const PassParams &P = *C.P;
 	const uint32_t lane = threadIdx.x & 31u, warp = G.thread() >> 5;
@@ -2740,15 +2737,23 @@ __device__ __forceinline__ void walk_list(const ShadeCtx &C, const DevInstance &
 		if (lane == 0)
 			L.rect[warp] = r;
 	}
+	if (RELOAD && !written)
+	{
+		G.sync();
+		chunk.load(G, mask, 0, I.mask_words, L);
+	}
 	for (uint32_t first = 0;;)
 	{
 		const bool last_chunk = first + T * LIST_WORDS >= I.mask_words;
 		for (uint32_t round = 0; round < chunk.total || (last_chunk && round == 0); round += CAP)
 		{
-			if (round)
+			if (!written)
+			{
+				if (round)
+					G.sync();
+				chunk.write(G, I.prim_lo, first, round, L);
 				G.sync();
-			chunk.write(G, I.prim_lo, first, round, L);
-			G.sync();
+			}
 			const uint32_t n = min(chunk.total - round, CAP);
 			const bool last_round = last_chunk && round + CAP >= chunk.total;
 			if constexpr (!AA)
@@ -2803,42 +2808,13 @@ __device__ __forceinline__ uint32_t subtile_mode(const PassParams &P, const DevI
 	return (I.rate_y_log2 != 0 && req) ? 2u : 1u;
 }
 
-// One sub-tile's pixel samples, NS per pixel, one thread per sample: the T
-// threads of the group have samples t (of 64 * NS) of it, as many as there are or
-// a part of them.  SS selects the super-sampled path.
-template <int NS, bool SS, bool AA, bool MIP, uint32_t T, uint32_t CAP>
-__device__ __forceinline__ void shade_subtile(const PassParams &P, const DevInstance &I, const ShadeGroup<T> &G,
-                                              const uint32_t *sub_masks, uint32_t sub, uint32_t t, ListShared<T, CAP> &list)
+// Samples t of the sub-tile at (sub_x, sub_y), one per thread of the group.
+template <int NS, bool SS, bool AA, bool MIP, bool RELOAD, uint32_t T, uint32_t CAP>
+__device__ __forceinline__ void shade_part(const PassParams &P, const DevInstance &I, const ShadeGroup<T> &G, const uint32_t *mask,
+                                           int32_t sub_x, int32_t sub_y, ListChunk<T, CAP> &chunk, bool written, uint32_t t,
+                                           ListShared<T, CAP> &list)
 {
-	const uint32_t gx = sub % I.sub_w, gy = sub / I.sub_w;
-	const uint32_t *mask = sub_masks + size_t(sub) * I.mask_words;
-
-	// What is the same for all warps is computed by one and waits for them at the
-	// list's barrier: sample offsets by the first, block addresses by the last
-	// (not for the two warps of a single-sampled sub-tile, where it costs more:
-	// plain frame 45.6 us without, 46.2 with; feedback frame at 8x 1.97 and 1.96 ms).
-	constexpr bool SHARE = T > 64u;
-	const int32_t sub_x = I.base_x + int32_t(gx * 8u), sub_y = I.base_y + int32_t(gy * 8u);
-	if (SS && G.thread() < NS)
-	{
-		int32_t x, y;
-		sample_offset(G.thread(), I.rate_x_log2, I.rate_y_log2, x, y);
-		list.smp[G.thread()] = make_int2(x << (3u - I.rate_y_log2), y << (3u - I.rate_y_log2));
-	}
-	if (SHARE && G.thread() >= T - 2u)
-	{
-		const bool z = G.thread() == T - 1u;
-		list.block[z ? 1 : 0] = swizzle_address(uint32_t(sub_x), uint32_t(sub_y), z ? I.zb_base : I.fb_base, I.fb_stride,
-		                                        z ? I.zb_psm : I.fb_psm);
-	}
-
-	// The list first: many sub-tiles of a pass of small primitives have none,
-	// and the samples' loads overlap its expansion.
-	ListChunk<T, CAP> chunk;
-	chunk.load(G, mask, 0, I.mask_words, list);
-	if (!chunk.total && I.mask_words <= T * LIST_WORDS)
-		return;
-
+	constexpr bool SHARE = T > 64u; // list.block is there
 	ShadeCtx C;
 	C.P = &P;
 	C.I = &I;
@@ -2943,7 +2919,7 @@ __device__ __forceinline__ void shade_subtile(const PassParams &P, const DevInst
 		S.depth = 0;
 
 	uint32_t covered = 0;
-	walk_list<NS, SS, AA, MIP, T, CAP>(C, I, G, mask, chunk, list, t, S, covered);
+	walk_list<NS, SS, AA, MIP, RELOAD, T, CAP>(C, I, G, mask, chunk, written, list, t, S, covered);
 
 	// walk_batch leaves nothing pending.
 	if (AA && S.pending.coverage > 0)
@@ -3060,22 +3036,75 @@ __device__ __forceinline__ void shade_subtile(const PassParams &P, const DevInst
 	}
 }
 
+// One sub-tile's pixel samples, NS per pixel, one thread per sample: the T
+// threads of the group have samples t (of 64 * NS) and, with PARTS, the samples T,
+// 2 T ... further on.  SS selects the super-sampled path.
+template <int NS, bool SS, bool AA, bool MIP, uint32_t PARTS, uint32_t T, uint32_t CAP>
+__device__ __forceinline__ void shade_subtile(const PassParams &P, const DevInstance &I, const ShadeGroup<T> &G,
+                                              const uint32_t *sub_masks, uint32_t sub, uint32_t t, ListShared<T, CAP> &list)
+{
+	const uint32_t gx = sub % I.sub_w, gy = sub / I.sub_w;
+	const uint32_t *mask = sub_masks + size_t(sub) * I.mask_words;
+
+	// What is the same for all warps is computed by one and waits for them at the
+	// list's barrier: sample offsets by the first, block addresses by the last
+	// (not for the two warps of a single-sampled sub-tile, where it costs more:
+	// plain frame 45.6 us without, 46.2 with; feedback frame at 8x 1.97 and 1.96 ms).
+	constexpr bool SHARE = T > 64u;
+	const int32_t sub_x = I.base_x + int32_t(gx * 8u), sub_y = I.base_y + int32_t(gy * 8u);
+	if (SS && G.thread() < NS)
+	{
+		int32_t x, y;
+		sample_offset(G.thread(), I.rate_x_log2, I.rate_y_log2, x, y);
+		list.smp[G.thread()] = make_int2(x << (3u - I.rate_y_log2), y << (3u - I.rate_y_log2));
+	}
+	if (SHARE && G.thread() >= T - 2u)
+	{
+		const bool z = G.thread() == T - 1u;
+		list.block[z ? 1 : 0] = swizzle_address(uint32_t(sub_x), uint32_t(sub_y), z ? I.zb_base : I.fb_base, I.fb_stride,
+		                                        z ? I.zb_psm : I.fb_psm);
+	}
+
+	// The list first: many sub-tiles of a pass of small primitives have none,
+	// and the samples' loads overlap its expansion.
+	ListChunk<T, CAP> chunk;
+	chunk.load(G, mask, 0, I.mask_words, list);
+	if (!chunk.total && I.mask_words <= T * LIST_WORDS)
+		return;
+	if constexpr (PARTS == 1)
+		shade_part<NS, SS, AA, MIP, false, T, CAP>(P, I, G, mask, sub_x, sub_y, chunk, false, t, list);
+	else
+	{
+		// Nearly every list fits: written once, and no barrier from there on.
+		const bool written = I.mask_words <= T * LIST_WORDS && chunk.total <= CAP;
+		if (written)
+		{
+			chunk.write(G, I.prim_lo, 0, 0, list);
+			G.sync();
+		}
+		#pragma unroll 1
+		for (uint32_t part = 0; part < PARTS; part++)
+			shade_part<NS, SS, AA, MIP, true, T, CAP>(P, I, G, mask, sub_x, sub_y, chunk, written, t + part * T, list);
+	}
+}
+
 // Indices held in shared memory at a time.
 constexpr uint32_t SHADE_LIST_CAP = 2048u, BATCH_LIST_CAP = 512u;
 
 // Sub-tiles whose coarse tile selects the other path exit immediately.
 template <int NS, bool SS, bool AA, bool MIP>
-__global__ void __launch_bounds__(ShadeCta<NS>::THREADS, PGS_SHADE_MIN_BLOCKS(NS, AA || MIP)) shade_kernel(PassParams P, DevInstance I, const uint32_t *sub_masks,
+__global__ void __launch_bounds__(ShadeCta<NS>::THREADS, PGS_SHADE_MIN_BLOCKS(NS)) shade_kernel(PassParams P, DevInstance I, const uint32_t *sub_masks,
                                                         const uint32_t *tile_flags)
 {
-	constexpr uint32_t T = ShadeCta<NS>::THREADS, PARTS = ShadeCta<NS>::PARTS;
+	constexpr uint32_t T = ShadeCta<NS>::THREADS;
 	__shared__ ListShared<T, SHADE_LIST_CAP> list;
-	const uint32_t sub = blockIdx.x / PARTS, part = blockIdx.x % PARTS;
+	const uint32_t sub = blockIdx.x;
 	if (sub >= I.sub_w * I.sub_h)
 		return;
 	if (subtile_mode(P, I, tile_flags, sub) != (SS ? 2u : 1u))
 		return;
-	shade_subtile<NS, SS, AA, MIP, T, SHADE_LIST_CAP>(P, I, ShadeGroup<T>{ 0u }, sub_masks, sub, part * T + threadIdx.x, list);
+	shade_subtile<NS, SS, AA, MIP, ShadeCta<NS>::PARTS, T, SHADE_LIST_CAP>(P, I, ShadeGroup<T>{ 0u }, sub_masks, sub, threadIdx.x,
+	                                                                       list);
 }
 
 // ---------------------------------------------------------------------------
@@ -3108,7 +3137,7 @@ template <int NS, bool SS, bool AA, uint32_t T>
 __device__ __noinline__ void shade_subtile_call(const PassParams &P, const DevInstance &I, const uint32_t *sub_masks, uint32_t sub,
                                                 uint32_t t, uint32_t bar, ListShared<T, BATCH_LIST_CAP> &list)
 {
-	shade_subtile<NS, SS, AA, false, T, BATCH_LIST_CAP>(P, I, ShadeGroup<T>{ bar }, sub_masks, sub, t, list);
+	shade_subtile<NS, SS, AA, false, 1, T, BATCH_LIST_CAP>(P, I, ShadeGroup<T>{ bar }, sub_masks, sub, t, list);
 }
 
 template <int BLOCK>
