@@ -785,7 +785,7 @@ struct CudaBackend
 					m.offset = uint32_t(texels);
 					uint32_t n = m.ext_u * m.ext_v;
 					texels += n;
-					max_texels = std::max(max_texels, n);
+					max_texels = std::max(max_texels, (m.ext_u + 3u) / 4u * m.ext_v); // threads of the decode
 				}
 				const TexImage &base_image = im[i * TEX_SLOTS];
 				for (uint32_t way = 0; way < 4; way++)
@@ -1226,7 +1226,7 @@ struct CudaBackend
 				c.src_vram = d_snapshot;
 			}
 			StageScope ts(this, PGS_TIMESTAMP_COPY_VRAM);
-			upload_kernel<<<dim3((c.width + 31) / 32, (c.height + 7) / 8), 256, 0, stream>>>(c, d_vram);
+			upload_kernel<<<dim3(upload_tiles_x(c), upload_tiles_y(c)), 256, 0, stream>>>(c, d_vram);
 			launch_counter++;
 			CUDA_TRY(cudaGetLastError());
 			return PGS_OK;
@@ -1322,7 +1322,7 @@ struct CudaBackend
 				c.host = d_arena + list[j].copy_host_off;
 				B.c[B.count] = c;
 				B.block_start[B.count] = blocks;
-				blocks += ((c.width + 31u) / 32u) * ((c.height + 7u) / 8u);
+				blocks += upload_tiles_x(c) * upload_tiles_y(c);
 				B.count++;
 				j++;
 			}
@@ -1897,7 +1897,7 @@ struct CudaBackend
 		}
 		{
 			StageScope ts(this, PGS_TIMESTAMP_READBACK);
-			const uint64_t threads = (R.size + 15u) / 16u;
+			const uint64_t threads = (R.size + 3u) / 4u;
 			readback_kernel<<<uint32_t((threads + 255u) / 256u), 256, 0, stream>>>(R, d_vram, d_readback);
 			launch_counter++;
 			CUDA_TRY(cudaGetLastError());

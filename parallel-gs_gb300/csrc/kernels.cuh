@@ -1209,10 +1209,24 @@ __device__ __forceinline__ const uint8_t *texture_source(const PassParams &P, ui
 	return P.vram;
 }
 
-__device__ __forceinline__ uint32_t fetch_texel(const PassParams &P, const uint8_t *v, const pgs_texture_desc &t,
-                                                uint32_t tbp, uint32_t tbw, int32_t x, int32_t y)
+// Address of pixel x + k of a row minus that of pixel x, x a multiple of 4: the
+// four lie in one block, and their two low coordinate bits go to address bits of
+// their own, clear in the first one's address.
+__device__ __forceinline__ uint32_t quad_offset(uint32_t psm, uint32_t k)
 {
-	uint32_t a = swizzle_address(uint32_t(x), uint32_t(y), tbp, tbw, t.psm);
+	const uint32_t lo = k & 1u, hi = (k >> 1) & 1u;
+	switch (psm)
+	{
+	case PSMCT16: case PSMCT16S: case PSMZ16: case PSMZ16S: return lo * 2u + hi * 8u; // halves
+	case PSMT8: return lo * 4u + hi * 16u;                                              // bytes
+	case PSMT4: return lo * 8u + hi * 32u;                                              // nibbles
+	default: return lo + hi * 4u;                                                       // words
+	}
+}
+
+// Texel at address a of the texture's format.
+__device__ __forceinline__ uint32_t fetch_texel(const PassParams &P, const uint8_t *v, const pgs_texture_desc &t, uint32_t a)
+{
 	switch (t.psm)
 	{
 	case PSMCT24: case PSMZ24:
@@ -1325,33 +1339,54 @@ __device__ __forceinline__ int32_t wrap_coord(int32_t v, uint32_t mode, uint32_t
 
 // Grid y = texture, z = slot (mip level, or sample layer of a super-sampled
 // texture); level l reads from MIPTBP's base and stride (upload_texture's
-// per-level loop, gs/gs_renderer.cpp:3543-3590).
+// per-level loop, gs/gs_renderer.cpp:3543-3590).  A thread decodes four texels of
+// a row, which share one address computation.
+// Bound: issue of the address and palette arithmetic, not the few bytes per texel
+// (eight 256x256 PSMT8 textures: a texel per thread 3.5 M warp instructions, so 1.9;
+// a light frame that decodes and uploads them 25.6 -> 22.8 us per replay).
 __global__ void __launch_bounds__(256) texture_decode_kernel(PassParams P)
 {
 	const uint32_t tex = blockIdx.y, level = blockIdx.z;
 	if (tex >= P.num_textures)
 		return;
-	const pgs_texture_desc t = P.textures[tex];
+	const pgs_texture_desc &t = P.textures[tex];
 	if (level >= texture_slots(t))
 		return;
 	const TexImage im = P.tex_images[tex * TEX_SLOTS + level];
+	const uint32_t quads = (im.ext_u + 3u) / 4u;
 	const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-	if (i >= im.ext_u * im.ext_v)
+	if (i >= quads * im.ext_v)
 		return;
-	const int32_t x = int32_t(i % im.ext_u), y = int32_t(i / im.ext_u);
+	const uint32_t x = i % quads * 4u, y = i / quads;
 	const uint8_t *src = texture_source(P, tex);
+	uint32_t *dst = P.texels + im.offset + y * im.ext_u + x;
+	const uint32_t n = min(im.ext_u - x, 4u);
+	uint32_t c[4] = {};
 	if (t.samples > 1 && level > 0)
 	{
-		P.texels[im.offset + i] = fetch_texel_sample(P, src, t, x, y, level - 1u);
-		return;
+		#pragma unroll
+		for (uint32_t k = 0; k < 4; k++)
+			if (k < n)
+				c[k] = fetch_texel_sample(P, src, t, int32_t(x + k), int32_t(y), level - 1u);
 	}
-	uint32_t tbp = t.tbp0, tbw = t.tbw;
-	if (level)
+	else
 	{
-		tbp = t.mip[level - 1] & 0x3fffu;
-		tbw = t.mip[level - 1] >> 16;
+		const uint32_t tbp = level ? t.mip[level - 1] & 0x3fffu : t.tbp0, tbw = level ? t.mip[level - 1] >> 16 : t.tbw;
+		const uint32_t a = swizzle_address(x, y, tbp, tbw, t.psm);
+		#pragma unroll
+		for (uint32_t k = 0; k < 4; k++)
+			if (k < n)
+				c[k] = fetch_texel(P, src, t, a + quad_offset(t.psm, k));
 	}
-	P.texels[im.offset + i] = fetch_texel(P, src, t, tbp, tbw, x, y);
+	if (!((im.offset | im.ext_u) & 3u))
+		*reinterpret_cast<uint4 *>(dst) = make_uint4(c[0], c[1], c[2], c[3]);
+	else
+	{
+		#pragma unroll
+		for (uint32_t k = 0; k < 4; k++)
+			if (k < n)
+				dst[k] = c[k];
+	}
 }
 
 // log2 of a positive normal float: ln m = 2 atanh(s), s = (m - 1) / (m + 1),
@@ -3523,55 +3558,121 @@ __device__ __forceinline__ uint32_t read_pixel(const uint8_t *vram, uint32_t psm
 	return v32[a];
 }
 
-__device__ __forceinline__ void upload_pixel(const CopyParams &C, uint8_t *vram, uint32_t x, uint32_t y)
+// Uploads go in tiles of 32 x 32 pixels from a multiple of 4 in the destination
+// on, a thread per four pixels of a row, which share one destination address
+// computation and, where they are aligned and all there, one payload load.
+// Bound: issue of the address arithmetic (eight 256x256 PSMT8 textures with their
+// palettes: a pixel per thread 4.7 M warp instructions, so 1.8).
+__host__ __device__ inline uint32_t upload_tiles_x(const CopyParams &C) { return ((C.dsax & 3u) + C.width + 31u) / 32u; }
+__host__ __device__ inline uint32_t upload_tiles_y(const CopyParams &C) { return (C.height + 31u) / 32u; }
+
+// Four pixels of the tile at (tx, ty).
+__device__ __forceinline__ void upload_quad(const CopyParams &C, uint8_t *vram, uint32_t tx, uint32_t ty)
 {
-	if (x >= C.width || y >= C.height)
+	// Pixel k of the quad is column x0 + k of the rectangle (x0 may be negative).
+	const int32_t x0 = int32_t(tx * 32u + (threadIdx.x & 7u) * 4u) - int32_t(C.dsax & 3u);
+	const uint32_t y = ty * 32u + (threadIdx.x >> 3);
+	if (y >= C.height || x0 >= int32_t(C.width))
 		return;
-	uint32_t eff_stride = C.dbw;
-	if (C.dpsm == PSMT4 || C.dpsm == PSMT8)
-		eff_stride &= ~1u;
-	if (x >= eff_stride * 64u)
+	uint32_t limit = C.width;
 	{
-		Layout L = psm_layout(C.dpsm);
-		uint32_t last = (C.dsay + C.height - 1u) >> L.ph, cur = (C.dsay + y) >> L.ph;
-		if (last != cur)
-			return;
+		// Columns past the buffer's stride are only written on the last page row.
+		uint32_t eff_stride = C.dbw;
+		if (C.dpsm == PSMT4 || C.dpsm == PSMT8)
+			eff_stride &= ~1u;
+		const Layout L = psm_layout(C.dpsm);
+		if ((C.dsay + C.height - 1u) >> L.ph != (C.dsay + y) >> L.ph)
+			limit = min(limit, eff_stride * 64u);
 	}
-	uint32_t dx = (x + C.dsax) & 2047u, dy = (y + C.dsay) & 2047u;
-	uint32_t data;
+	const uint32_t dx = uint32_t(x0 + int32_t(C.dsax)) & 2047u, dy = (y + C.dsay) & 2047u;
+	uint32_t data[4];
+	uint32_t have = 0; // pixels to write
 	if (C.xdir == HOST_TO_LOCAL)
 	{
-		uint64_t sa = uint64_t(y) * C.width + x;
-		uint32_t b = psm_bits_per_pixel(C.dpsm);
-		uint64_t factor = (b == 32 || b == 24) ? 2 : (b == 16 ? 4 : (b == 8 ? 8 : 16));
-		uint64_t avail = b == 32 ? C.host_size / 4 : (b == 24 ? C.host_size / 3 : (b == 16 ? C.host_size / 2 : (b == 8 ? C.host_size : 2 * C.host_size)));
-		if (sa * factor < C.host_offset_qwords || sa >= avail)
+		const uint32_t b = psm_bits_per_pixel(C.dpsm);
+		const uint32_t factor = (b == 32 || b == 24) ? 2 : (b == 16 ? 4 : (b == 8 ? 8 : 16));
+		const uint64_t avail = b == 32 ? C.host_size / 4 : (b == 24 ? C.host_size / 3 : (b == 16 ? C.host_size / 2 : (b == 8 ? C.host_size : 2 * C.host_size)));
+		const uint32_t row = y * C.width;
+		#pragma unroll
+		for (int k = 0; k < 4; k++)
+		{
+			const int32_t x = x0 + k;
+			const uint64_t sa = uint64_t(row) + uint32_t(x);
+			if (x >= 0 && uint32_t(x) < limit && sa * factor >= C.host_offset_qwords && sa < avail)
+				have |= 1u << k;
+		}
+		if (!have)
 			return;
-		// The payload starts 256-byte aligned: a warp's 32 consecutive pixels
-		// read one contiguous span, with one load of the pixel's width each.
+		// The payload starts 256-byte aligned.
 		const uint8_t *h = C.host;
-		if (b == 24) data = uint32_t(h[3 * sa]) | (uint32_t(h[3 * sa + 1]) << 8) | (uint32_t(h[3 * sa + 2]) << 16);
-		else if (b == 16) data = reinterpret_cast<const uint16_t *>(h)[sa];
-		else if (b == 8) data = h[sa];
-		else if (b == 4) data = (uint32_t(h[sa >> 1]) >> ((sa & 1) * 4)) & 15u;
-		else data = reinterpret_cast<const uint32_t *>(h)[sa];
+		const uint32_t sa = row + uint32_t(x0); // of pixel 0, if it is there
+		if (have == 15u && !(sa & 3u) && (b == 32 || b == 16 || b == 8))
+		{
+			if (b == 32)
+			{
+				const uint4 v = *reinterpret_cast<const uint4 *>(h + size_t(sa) * 4u);
+				data[0] = v.x; data[1] = v.y; data[2] = v.z; data[3] = v.w;
+			}
+			else if (b == 16)
+			{
+				const uint2 v = *reinterpret_cast<const uint2 *>(h + size_t(sa) * 2u);
+				data[0] = v.x & 0xffffu; data[1] = v.x >> 16; data[2] = v.y & 0xffffu; data[3] = v.y >> 16;
+			}
+			else
+			{
+				const uint32_t v = *reinterpret_cast<const uint32_t *>(h + sa);
+				data[0] = v & 0xffu; data[1] = (v >> 8) & 0xffu; data[2] = (v >> 16) & 0xffu; data[3] = v >> 24;
+			}
+		}
+		else
+		{
+			#pragma unroll
+			for (int k = 0; k < 4; k++)
+			{
+				if (!((have >> k) & 1u))
+					continue;
+				const size_t p = size_t(row) + uint32_t(x0 + k);
+				if (b == 24) data[k] = uint32_t(h[3 * p]) | (uint32_t(h[3 * p + 1]) << 8) | (uint32_t(h[3 * p + 2]) << 16);
+				else if (b == 16) data[k] = reinterpret_cast<const uint16_t *>(h)[p];
+				else if (b == 8) data[k] = h[p];
+				else if (b == 4) data[k] = (uint32_t(h[p >> 1]) >> ((p & 1) * 4)) & 15u;
+				else data[k] = reinterpret_cast<const uint32_t *>(h)[p];
+			}
+		}
 	}
 	else
 	{
-		uint32_t sx = (x + C.ssax) & 2047u, sy = (y + C.ssay) & 2047u;
-		data = read_pixel(C.src_vram, C.spsm, swizzle_address(sx, sy, C.sbp, C.sbw, C.spsm));
+		// One address for all four where the source is as aligned as the destination.
+		const uint32_t sy = (y + C.ssay) & 2047u;
+		const bool aligned = !((C.ssax ^ C.dsax) & 3u);
+		const uint32_t sa = swizzle_address(uint32_t(x0 + int32_t(C.ssax)) & 2047u, sy, C.sbp, C.sbw, C.spsm);
+		#pragma unroll
+		for (int k = 0; k < 4; k++)
+		{
+			const int32_t x = x0 + k;
+			if (x < 0 || uint32_t(x) >= limit)
+				continue;
+			const uint32_t s = aligned ? sa + quad_offset(C.spsm, uint32_t(k))
+			                           : swizzle_address((uint32_t(x) + C.ssax) & 2047u, sy, C.sbp, C.sbw, C.spsm);
+			data[k] = read_pixel(C.src_vram, C.spsm, s);
+			have |= 1u << k;
+		}
 	}
-	write_pixel(vram, C.dpsm, swizzle_address(dx, dy, C.dbp, C.dbw, C.dpsm), data, C.invalidate_ss != 0);
+	const uint32_t a = swizzle_address(dx, dy, C.dbp, C.dbw, C.dpsm);
+	#pragma unroll
+	for (int k = 0; k < 4; k++)
+		if ((have >> k) & 1u)
+			write_pixel(vram, C.dpsm, a + quad_offset(C.dpsm, uint32_t(k)), data[k], C.invalidate_ss != 0);
 }
 
 __global__ void __launch_bounds__(256) upload_kernel(CopyParams C, uint8_t *vram)
 {
-	upload_pixel(C, vram, blockIdx.x * 32u + (threadIdx.x & 31u), blockIdx.y * 8u + (threadIdx.x >> 5));
+	upload_quad(C, vram, blockIdx.x, blockIdx.y);
 }
 
 // Consecutive host->local uploads whose destination blocks do not overlap, in
-// one launch: the order among them cannot change VRAM.  Blocks of 32 x 8
-// pixels are dealt out to the uploads by block_start.
+// one launch: the order among them cannot change VRAM.  Tiles are dealt out to the
+// uploads by block_start.
 constexpr uint32_t UPLOAD_BATCH_MAX = 16;
 struct UploadBatch
 {
@@ -3586,14 +3687,15 @@ __global__ void __launch_bounds__(256) upload_batch_kernel(UploadBatch B, uint8_
 	while (i + 1u < B.count && blockIdx.x >= B.block_start[i + 1])
 		i++;
 	const CopyParams &C = B.c[i];
-	const uint32_t local = blockIdx.x - B.block_start[i], bw = (C.width + 31u) / 32u;
-	upload_pixel(C, vram, (local % bw) * 32u + (threadIdx.x & 31u), (local / bw) * 8u + (threadIdx.x >> 5));
+	const uint32_t local = blockIdx.x - B.block_start[i], tiles_x = upload_tiles_x(C);
+	upload_quad(C, vram, local % tiles_x, local / tiles_x);
 }
 
 // LOCAL->HOST read-out of a rectangle of plane 0 into linear bytes
 // (vram_readback, gs/gs_util.hpp:50-110): pixels in row order at their host
-// size (4, 3, 2 or 1 bytes).  Each thread packs 16 consecutive output bytes
-// and writes them as one 16-byte store where the output allows.
+// size (4, 3, 2 or 1 bytes).  Each thread packs 4 consecutive output bytes and
+// writes them as one word where the output allows.  Bound: latency; 16 bytes a
+// thread left a 64 KB rectangle on 16 CTAs (9.8 us, so 5.0).
 struct ReadbackParams
 {
 	uint32_t sbp, sbw, spsm, ssax, ssay, width, height, bytes_per_pixel;
@@ -3614,7 +3716,7 @@ __device__ __forceinline__ uint32_t readback_fetch(uint32_t spsm, const uint8_t 
 
 __global__ void __launch_bounds__(256) readback_kernel(ReadbackParams R, const uint8_t *vram, uint8_t *out)
 {
-	const uint64_t first = (uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) * 16u;
+	const uint64_t first = (uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) * 4u;
 	if (first >= R.size)
 		return;
 	const uint32_t B = R.bytes_per_pixel;
@@ -3636,19 +3738,13 @@ __global__ void __launch_bounds__(256) readback_kernel(ReadbackParams R, const u
 		}
 		return v;
 	};
-	if (first + 16u <= R.size)
+	if (first + 4u <= R.size)
 	{
-		uint32_t w[4];
+		uint32_t v = 0;
 		#pragma unroll
-		for (int q = 0; q < 4; q++)
-		{
-			uint32_t v = 0;
-			#pragma unroll
-			for (int b = 0; b < 4; b++)
-				v |= next() << (8 * b);
-			w[q] = v;
-		}
-		*reinterpret_cast<uint4 *>(out + first) = make_uint4(w[0], w[1], w[2], w[3]);
+		for (int b = 0; b < 4; b++)
+			v |= next() << (8 * b);
+		*reinterpret_cast<uint32_t *>(out + first) = v;
 	}
 	else
 		for (uint64_t b = first; b < R.size; b++)
