@@ -57,6 +57,12 @@ __constant__ int d_pad_out[LAYERS] = { 32, 32, 32, 32, 32, 8 };
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) { return uint32_t(__cvta_generic_to_shared(p)); }
 
+// 16 bytes from global to shared memory, or zeros.
+__device__ __forceinline__ void cp_async16(void *dst, const void *src, bool valid)
+{
+	asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(smem_u32(dst)), "l"(src), "r"(valid ? 16 : 0) : "memory");
+}
+
 __device__ __forceinline__ void ldsm_x4(uint32_t addr, uint32_t &r0, uint32_t &r1, uint32_t &r2, uint32_t &r3)
 {
 	asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n"
@@ -92,6 +98,30 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi)
 {
 	__nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
 	return *reinterpret_cast<uint32_t *>(&v);
+}
+
+// A pixel of a caller's image, which may start at any byte.
+__device__ __forceinline__ uint32_t load_pixel(const uint8_t *p)
+{
+	if (!(reinterpret_cast<uintptr_t>(p) & 3u))
+		return *reinterpret_cast<const uint32_t *>(p);
+	return uint32_t(p[0]) | (uint32_t(p[1]) << 8) | (uint32_t(p[2]) << 16) | (uint32_t(p[3]) << 24);
+}
+
+__device__ __forceinline__ void store_pixel(uint8_t *p, uint32_t c)
+{
+	if (!(reinterpret_cast<uintptr_t>(p) & 3u))
+		*reinterpret_cast<uint32_t *>(p) = c;
+	else
+		for (int k = 0; k < 4; k++)
+			p[k] = uint8_t(c >> (8 * k));
+}
+
+// The two BF16 values of v where those of m are positive, else 0.
+__device__ __forceinline__ uint32_t mask_positive(uint32_t v, uint32_t m)
+{
+	const float lo = __uint_as_float(m << 16), hi = __uint_as_float(m & 0xffff0000u);
+	return (lo > 0.0f ? v & 0xffffu : 0u) | (hi > 0.0f ? v & 0xffff0000u : 0u);
 }
 
 // One RGBA8 pixel as the network's first four input channels (x / 255 in
@@ -140,13 +170,24 @@ struct ConvArgs
 };
 
 // Grid: (ceil(W/16), ceil(H/16), N); 256 threads.
+// Rows of 32 channels have their 16-byte chunks exchanged by bits of the row, rows
+// of 16 are padded by 8 channels: either way eight rows read by ldmatrix lie in
+// different banks.  Without padding eight CTAs of the last layer fit an SM, one
+// wave of a 640x448 frame.
+// Bound: latency (halo loads, barrier, fragment loads, one tile per CTA).  Network
+// on one 640x448 frame: outputs staged for 16-byte stores and whole pixels 69.6 ->
+// 69.1 us, halo by asynchronous copies and eight CTAs per SM -> 64.7.
 template <int CIN, int COUT, int EPI>
-__global__ void __launch_bounds__(256) conv3x3_kernel(ConvArgs A)
+__global__ void __launch_bounds__(256, EPI == EPI_LAST ? 8 : 4) conv3x3_kernel(ConvArgs A)
 {
-	constexpr int PS = CIN + 8;        // padded pixel stride (elements): conflict-free ldmatrix rows
+	constexpr int PS = CIN == 32 ? 32 : CIN + 8; // row stride (elements)
+	auto at = [](int row, int chunk) { return CIN == 32 ? row * PS + ((chunk ^ (row >> 1)) & 3) * 8 : row * PS + chunk * 8; };
 	constexpr int NT = COUT / 8;       // n8 tiles
-	__shared__ __align__(16) __nv_bfloat16 s_in[HALO * HALO * PS];
-	__shared__ __align__(16) __nv_bfloat16 s_w[9 * COUT * PS];
+	constexpr int OS = COUT + 8;       // padded pixel stride of the staged output
+	constexpr int IN = HALO * HALO * PS, OUT = EPI == EPI_LAST ? 0 : TILE * TILE * OS;
+	// Input halo and weights; then, in their place, the tile's output.
+	__shared__ __align__(16) __nv_bfloat16 s_buf[IN + 9 * COUT * PS > OUT ? IN + 9 * COUT * PS : OUT];
+	__nv_bfloat16 *s_in = s_buf, *s_w = s_buf + IN;
 
 	const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 	const int x0 = blockIdx.x * TILE, y0 = blockIdx.y * TILE, img = blockIdx.z;
@@ -156,10 +197,7 @@ __global__ void __launch_bounds__(256) conv3x3_kernel(ConvArgs A)
 	// for the previous layer, then its output.
 	constexpr int CH = CIN / 8;
 	for (int i = tid; i < 9 * COUT * CH; i += 256)
-	{
-		int r = i / CH, c = (i % CH) * 8;
-		*reinterpret_cast<uint4 *>(s_w + r * PS + c) = *reinterpret_cast<const uint4 *>(A.wt + r * CIN + c);
-	}
+		*reinterpret_cast<uint4 *>(s_w + at(i / CH, i % CH)) = *reinterpret_cast<const uint4 *>(A.wt + size_t(i) * 8);
 	griddep_wait();
 
 	// Input halo, 16-byte chunks, zero outside the image.
@@ -182,13 +220,17 @@ __global__ void __launch_bounds__(256) conv3x3_kernel(ConvArgs A)
 	else
 	for (int i = tid; i < HALO * HALO * CH; i += 256)
 	{
-		int p = i / CH, c = (i % CH) * 8;
+		int p = i / CH, c = i % CH;
 		int gx = x0 - 1 + p % HALO, gy = y0 - 1 + p / HALO;
-		uint4 v = make_uint4(0, 0, 0, 0);
-		if (gx >= 0 && gy >= 0 && gx < A.w && gy < A.h)
-			v = *reinterpret_cast<const uint4 *>(A.in + ((size_t(img) * A.h + gy) * A.w + gx) * CIN + c);
-		*reinterpret_cast<uint4 *>(s_in + p * PS + c) = v;
+		const bool in = gx >= 0 && gy >= 0 && gx < A.w && gy < A.h;
+		const __nv_bfloat16 *src = A.in + ((size_t(img) * A.h + gy) * A.w + gx) * CIN + c * 8;
+		if constexpr (CIN == 32)
+			cp_async16(s_in + at(p, c), in ? src : A.in, in);
+		else
+			*reinterpret_cast<uint4 *>(s_in + at(p, c)) = in ? *reinterpret_cast<const uint4 *>(src) : make_uint4(0, 0, 0, 0);
 	}
+	if constexpr (CIN == 32)
+		asm volatile("cp.async.wait_all;\n" ::: "memory");
 	__syncthreads();
 
 	float acc[2][NT][4];
@@ -212,7 +254,7 @@ __global__ void __launch_bounds__(256) conv3x3_kernel(ConvArgs A)
 			for (int r = 0; r < 2; r++)
 			{
 				int py = warp * 2 + r + dy, px = (lane & 15) + dx;
-				const __nv_bfloat16 *p = s_in + (py * HALO + px) * PS + kc * 16 + (lane >> 4) * 8;
+				const __nv_bfloat16 *p = s_in + at(py * HALO + px, kc * 2 + (lane >> 4));
 				ldsm_x4(smem_u32(p), a[r][0], a[r][1], a[r][2], a[r][3]);
 			}
 			#pragma unroll
@@ -222,7 +264,7 @@ __global__ void __launch_bounds__(256) conv3x3_kernel(ConvArgs A)
 				{
 					// Two n-tiles: lanes 0-15 tile j (k 0-7, 8-15), 16-31 tile j+1.
 					int nt = j + (lane >> 4), nrow = nt * 8 + (lane & 7), kh = (lane >> 3) & 1;
-					const __nv_bfloat16 *p = s_w + (tap * COUT + nrow) * PS + kc * 16 + kh * 8;
+					const __nv_bfloat16 *p = s_w + at(tap * COUT + nrow, kc * 2 + kh);
 					uint32_t b0, b1, b2, b3;
 					ldsm_x4(smem_u32(p), b0, b1, b2, b3);
 					#pragma unroll
@@ -235,7 +277,7 @@ __global__ void __launch_bounds__(256) conv3x3_kernel(ConvArgs A)
 				else
 				{
 					int nrow = j * 8 + (lane & 7), kh = (lane >> 3) & 1;
-					const __nv_bfloat16 *p = s_w + (tap * COUT + nrow) * PS + kc * 16 + kh * 8;
+					const __nv_bfloat16 *p = s_w + at(tap * COUT + nrow, kc * 2 + kh);
 					uint32_t b0, b1;
 					ldsm_x2(smem_u32(p), b0, b1);
 					#pragma unroll
@@ -248,53 +290,74 @@ __global__ void __launch_bounds__(256) conv3x3_kernel(ConvArgs A)
 
 	// Epilogue: thread holds rows g, g+8 and columns 2t, 2t+1 of each tile.
 	const int g = lane >> 2, t = lane & 3;
-	#pragma unroll
-	for (int r = 0; r < 2; r++)
+	if constexpr (EPI == EPI_LAST)
 	{
-		const int gy = y0 + warp * 2 + r;
+		// Residual over the input image in [0, 1]: the first lane of four has
+		// channels 0 and 1, takes 2 and 3 from the next and stores the pixel.
 		#pragma unroll
-		for (int half = 0; half < 2; half++)
+		for (int r = 0; r < 2; r++)
+			#pragma unroll
+			for (int half = 0; half < 2; half++)
+			{
+				float v[4] = { acc[r][0][half * 2], acc[r][0][half * 2 + 1] };
+				v[2] = __shfl_down_sync(0xffffffffu, v[0], 1);
+				v[3] = __shfl_down_sync(0xffffffffu, v[1], 1);
+				const int gx = x0 + g + half * 8, gy = y0 + warp * 2 + r;
+				if (t != 0 || gx >= A.w || gy >= A.h)
+					continue;
+				const size_t pix = (size_t(img) * A.h + gy) * A.w + gx;
+				const uint32_t c = reinterpret_cast<const uint32_t *>(A.image)[pix];
+				uint32_t packed = 0;
+				#pragma unroll
+				for (int k = 0; k < 4; k++)
+				{
+					v[k] = v[k] + A.bias[k] + float((c >> (8 * k)) & 0xffu) / 255.0f;
+					packed |= uint32_t(rintf(fminf(fmaxf(v[k], 0.0f), 1.0f) * 255.0f)) << (8 * k);
+				}
+				if (A.out_f32)
+					reinterpret_cast<float4 *>(A.out_f32)[pix] = make_float4(v[0], v[1], v[2], v[3]);
+				if (A.out_rgba)
+					store_pixel(A.out_rgba + pix * 4, packed);
+			}
+	}
+	else
+	{
+		// Through shared memory, so that global memory sees 16 bytes a lane and
+		// whole sectors (4 bytes a lane, 16 of each 32-byte sector, otherwise).
+		__syncthreads();
+		#pragma unroll
+		for (int r = 0; r < 2; r++)
+			#pragma unroll
+			for (int half = 0; half < 2; half++)
+				#pragma unroll
+				for (int j = 0; j < NT; j++)
+				{
+					const int co = j * 8 + 2 * t;
+					float v0 = acc[r][j][half * 2], v1 = acc[r][j][half * 2 + 1];
+					if (EPI == EPI_RELU)
+					{
+						v0 = fmaxf(v0 + A.bias[co], 0.0f);
+						v1 = fmaxf(v1 + A.bias[co + 1], 0.0f);
+					}
+					*reinterpret_cast<uint32_t *>(s_buf + ((warp * 2 + r) * TILE + g + half * 8) * OS + co) = pack_bf16x2(v0, v1);
+				}
+		__syncthreads();
+		constexpr int CHUNKS = COUT / 8;
+		#pragma unroll
+		for (int i = tid; i < TILE * TILE * CHUNKS; i += 256)
 		{
-			const int gx = x0 + g + half * 8;
+			const int p = i / CHUNKS, c = (i % CHUNKS) * 8;
+			const int gx = x0 + p % TILE, gy = y0 + p / TILE;
 			if (gx >= A.w || gy >= A.h)
 				continue;
-			const size_t pix = (size_t(img) * A.h + gy) * A.w + gx;
-			#pragma unroll
-			for (int j = 0; j < NT; j++)
+			const size_t at = ((size_t(img) * A.h + gy) * A.w + gx) * COUT + c;
+			uint4 v = *reinterpret_cast<const uint4 *>(s_buf + p * OS + c);
+			if (EPI == EPI_MASK)
 			{
-				const int co = j * 8 + 2 * t;
-				float v0 = acc[r][j][half * 2], v1 = acc[r][j][half * 2 + 1];
-				if (EPI == EPI_RELU)
-				{
-					v0 = fmaxf(v0 + A.bias[co], 0.0f);
-					v1 = fmaxf(v1 + A.bias[co + 1], 0.0f);
-					*reinterpret_cast<uint32_t *>(A.out + pix * COUT + co) = pack_bf16x2(v0, v1);
-				}
-				else if (EPI == EPI_MASK)
-				{
-					__nv_bfloat162 m = *reinterpret_cast<const __nv_bfloat162 *>(A.mask + pix * COUT + co);
-					v0 = __bfloat162float(m.x) > 0.0f ? v0 : 0.0f;
-					v1 = __bfloat162float(m.y) > 0.0f ? v1 : 0.0f;
-					*reinterpret_cast<uint32_t *>(A.out + pix * COUT + co) = pack_bf16x2(v0, v1);
-				}
-				else if (co < 4)
-				{
-					// Residual over the input image in [0, 1].
-					float i0 = float(A.image[pix * 4 + co]) / 255.0f, i1 = float(A.image[pix * 4 + co + 1]) / 255.0f;
-					v0 = v0 + A.bias[co] + i0;
-					v1 = v1 + A.bias[co + 1] + i1;
-					if (A.out_f32)
-					{
-						A.out_f32[pix * 4 + co] = v0;
-						A.out_f32[pix * 4 + co + 1] = v1;
-					}
-					if (A.out_rgba)
-					{
-						A.out_rgba[pix * 4 + co] = uint8_t(rintf(fminf(fmaxf(v0, 0.0f), 1.0f) * 255.0f));
-						A.out_rgba[pix * 4 + co + 1] = uint8_t(rintf(fminf(fmaxf(v1, 0.0f), 1.0f) * 255.0f));
-					}
-				}
+				const uint4 m = *reinterpret_cast<const uint4 *>(A.mask + at);
+				v = make_uint4(mask_positive(v.x, m.x), mask_positive(v.y, m.y), mask_positive(v.z, m.z), mask_positive(v.w, m.w));
 			}
+			*reinterpret_cast<uint4 *>(A.out + at) = v;
 		}
 	}
 }
@@ -329,12 +392,6 @@ template <int CIN, int COUT>
 __host__ __device__ constexpr size_t wgrad_buffer_bytes()
 {
 	return (HALO * HALO * (CIN + 8) + TILE * TILE * (COUT + 8)) * 2;
-}
-
-// 16 bytes from global to shared memory, or zeros.
-__device__ __forceinline__ void cp_async16(void *dst, const void *src, bool valid)
-{
-	asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(smem_u32(dst)), "l"(src), "r"(valid ? 16 : 0) : "memory");
 }
 
 template <int CIN, int COUT>
@@ -511,7 +568,7 @@ __global__ void __launch_bounds__(256) loss_kernel(const float *out, const uint8
 	for (size_t p = size_t(blockIdx.x) * 256 + threadIdx.x; p < pixels; p += size_t(gridDim.x) * 256)
 	{
 		const float4 v = reinterpret_cast<const float4 *>(out)[p];
-		const uint32_t c = reinterpret_cast<const uint32_t *>(target)[p];
+		const uint32_t c = load_pixel(target + p * 4);
 		const float d[4] = { v.x - float(c & 0xffu) / 255.0f, v.y - float((c >> 8) & 0xffu) / 255.0f,
 		                     v.z - float((c >> 16) & 0xffu) / 255.0f, v.w - float(c >> 24) / 255.0f };
 		#pragma unroll
@@ -1292,7 +1349,7 @@ struct Upscaler
 				// 32 -> 4 likewise (N = 32 with 28 zero output channels).
 				k.out = nullptr;
 				k.image = d_img;
-				k.out_f32 = d_out;
+				k.out_f32 = keep_input || !out_rgba ? d_out : nullptr; // training reads it
 				k.out_rgba = out_rgba;
 				r = conv<32, 8, EPI_LAST>(k, !keep_input);
 			}

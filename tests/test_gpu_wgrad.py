@@ -57,3 +57,25 @@ def test_repeated_images_sum_over_all_tiles():
     _, many = gradient(np.repeat(img, 32, 0), np.repeat(tgt, 32, 0), p)
     for a, b in zip(layers(many), layers(one)):
         assert np.linalg.norm(a - b) < 1e-3 * np.linalg.norm(b)
+
+
+def test_targets_and_outputs_at_any_byte():
+    """Target and output images need no alignment (the input's is four bytes)."""
+    import torch
+    img, tgt = images(9, 2, 21, 19)
+    p = pgs.upscaler_init_params(9)
+    loss, g = gradient(img, tgt, p)
+    up = pgs.Upscaler(0)
+    try:
+        up.set_params(p)
+        di = torch.from_numpy(img).cuda()
+        odd = torch.empty(img.size + 1, dtype=torch.uint8, device="cuda")[1:]
+        odd.copy_(torch.from_numpy(tgt.reshape(-1)).cuda())
+        assert abs(up.backward(di, odd.view(img.shape)) - loss) <= 1e-12 * loss
+        even = torch.empty_like(di)
+        up.forward(di, even)
+        up.forward(di, odd.view(img.shape))
+        up.synchronize()
+        assert torch.equal(even.view(-1), odd)
+    finally:
+        up.close()
