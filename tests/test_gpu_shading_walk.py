@@ -177,3 +177,20 @@ def test_batched_rounds(cta_threads):
         batch.close()
         for be in backends:
             be.close()
+
+
+@pytest.mark.parametrize("ss", [1, 8, 16])
+def test_lists_of_several_chunks(ss):
+    """33,000 primitives: more than 1024 mask words, so lists come in chunks, also
+    where a CTA runs several parts of a sub-tile."""
+    rng = np.random.default_rng(ss)
+    s = gsgen.GifStream()
+    setup(s, gsgen.PSMCT32, gsgen.PSMZ24)
+    n = 33000
+    x = rng.integers(0, W * 16, size=(n, 1)) + rng.integers(-40, 41, size=(n, 3))
+    y = rng.integers(0, H * 16, size=(n, 1)) + rng.integers(-40, 41, size=(n, 3))
+    q = np.zeros((n * 3, 2, 2), dtype=np.uint64)
+    q[:, 0] = gsgen.q_rgbaq(rng.integers(0, 256, size=(n * 3, 4), dtype=np.int64))
+    q[:, 1] = gsgen.q_xyz2(np.clip(x, 0, W * 16).reshape(-1), np.clip(y, 0, H * 16).reshape(-1), rng.integers(0, 1 << 24, size=n * 3))
+    s.packed(gsgen.prim_reg(gsgen.PRIM_TRI, iip=1), [gsgen.D_RGBAQ, gsgen.D_XYZ2], q.reshape(-1, 2))
+    assert_same(*run_both(frame(s, ss, True, n)))
