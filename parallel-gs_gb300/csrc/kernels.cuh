@@ -2,13 +2,15 @@
 //
 //   setup_kernel     one thread per primitive: edge planes, reciprocal area,
 //                    attribute deltas, bounding box (triangle_setup.comp)
-//   bin_kernel       32 primitives per CTA: per-coarse-tile membership and
-//                    super-sampling flags (binning.comp), and the primitive's
-//                    bit in the bitmask of every 8x8 sub-tile it may touch;
-//                    the bitmask keeps primitive order without any sort
+//   bin_kernel       32 primitives per group, 1 to 16 CTAs each: per-coarse-tile
+//                    membership and super-sampling flags (binning.comp), and
+//                    the primitive's bit in the bitmask of every 8x8 sub-tile
+//                    it may touch; the bitmask keeps primitive order without
+//                    any sort
 //   shade_kernel     one CTA per 8x8-pixel sub-tile of a coarse tile, one
-//                    thread per pixel sample; walks the tile's primitives in
-//                    order with the deferred-shading logic of ubershader.comp
+//                    thread per pixel sample (256 threads at most, the rest
+//                    in turn); walks the tile's primitives in order with the
+//                    deferred-shading logic of ubershader.comp
 //   upload_kernel    host->local and local->local transfers into swizzled VRAM
 //   clut_kernel      CLUT instance load (clut_write.comp)
 //
@@ -983,15 +985,14 @@ __device__ __forceinline__ bool intersects_tile(const PrimSetup &s, int32_t lo0,
 // membership test and super-sampling flags (binning.comp:74-125); shading
 // lists are kept per 8x8 sub-tile as bitmasks over the pass's primitive range
 // so that ascending primitive order needs no sort.  The primitives of one mask
-// word (32) are a group; its
-// (primitive, tile) candidates, those of the coarse grid and then those of the
+// word (32) are a group; its (primitive, tile) candidates, those of the coarse grid and then those of the
 // sub-tile grid, are dealt out 32 at a time to the warps of gridDim.y CTAs, so
 // that neither a primitive over the whole frame nor one over hundreds of coarse
 // tiles holds a lane.
 // Bound: latency (dependent loads, shuffles and reductions at under 20 % of the
 // issue slots), hence many short chains: with one lane walking all coarse tiles
 // of its primitive and one CTA per group, a 61-primitive frame with a clear of
-// the whole frame took 47 us here and takes 4; the feedback frame's passes at 8x went from 15 to 4.6
+// the whole frame took 47 us here and takes 4; a feedback frame's passes at 8x went from 15 to 4.6.
 constexpr uint32_t BIN_GROUP_WARPS = 4;
 // CTAs a launch aims at when its groups are fewer (four per SM), up to 16 per group.
 constexpr uint32_t BIN_TARGET_CTAS = 608;

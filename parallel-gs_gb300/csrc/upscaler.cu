@@ -12,9 +12,10 @@
 //   layers 1-4: 32 -> 32, ReLU
 //   layer 5: 32 -> 4 (padded to 8), output = input + conv
 //
-// The same kernel computes the data gradient (flipped, transposed weights;
-// the epilogue multiplies by the ReLU mask of the layer below), and a second
-// kernel the weight gradient (K = pixels).
+// The 32 -> 32 layers run on tcgen05 (conv32_tc_kernel, further down) unless the
+// tensor path is switched off.  The same kernels compute the data gradient
+// (flipped, transposed weights; the epilogue multiplies by the ReLU mask of the
+// layer below), and another the weight gradient (K = pixels).
 #include "pgs.h"
 #include "umma.cuh"
 
