@@ -2669,7 +2669,6 @@ struct ListShared
 	uint32_t count[LIST_WORDS * T / 32u]; // per word of the chunk and warp
 	int2 smp[16];                         // sample offsets of WarpPlace
 	uint32_t block[2];                    // colour and depth address of the sub-tile's first pixel
-	int4 rect[T / 32u];                   // per warp, AA1 variants
 };
 
 // The T threads that run a sub-tile together: thread 0 of them is aligned to T,
@@ -2748,10 +2747,11 @@ __device__ __forceinline__ void walk_list(const ShadeCtx &C, const DevInstance &
                                           SampleState &S, uint32_t &covered)
 {
 	const PassParams &P = *C.P;
-	const uint32_t lane = threadIdx.x & 31u, warp = G.thread() >> 5;
+	const uint32_t lane = threadIdx.x & 31u;
 	const unsigned full = 0xffffffffu;
 	WarpPlace W;
 	uint32_t my_bit = 0, even_rows = 0, even_pixels = 0;
+	int4 rect = {}; // of the warp's raster positions, the same in every lane
 	if constexpr (!AA)
 	{
 		using B = WarpBlock<NS>;
@@ -2769,10 +2769,8 @@ __device__ __forceinline__ void walk_list(const ShadeCtx &C, const DevInstance &
 	else
 	{
 		const int32_t x0 = S.hx & C.snap_mask_x, y0 = S.hy & C.snap_mask_x & C.snap_mask_y;
-		const int4 r = make_int4(__reduce_min_sync(full, x0), __reduce_min_sync(full, y0),
-		                         __reduce_max_sync(full, S.hx), __reduce_max_sync(full, S.hy));
-		if (lane == 0)
-			L.rect[warp] = r;
+		rect = make_int4(__reduce_min_sync(full, x0), __reduce_min_sync(full, y0), __reduce_max_sync(full, S.hx),
+		                 __reduce_max_sync(full, S.hy));
 	}
 	if (RELOAD && !written)
 	{
@@ -2809,7 +2807,7 @@ __device__ __forceinline__ void walk_list(const ShadeCtx &C, const DevInstance &
 				if (k < n)
 				{
 					pi = L.ids[k];
-					hit = may_cover(P.setup[pi], P.prims[pi].state, L.rect[warp], C.dim);
+					hit = may_cover(P.setup[pi], P.prims[pi].state, rect, C.dim);
 				}
 				uint32_t bits = __ballot_sync(full, hit);
 				while (bits)
