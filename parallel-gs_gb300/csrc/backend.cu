@@ -1226,7 +1226,7 @@ struct CudaBackend
 				c.src_vram = d_snapshot;
 			}
 			StageScope ts(this, PGS_TIMESTAMP_COPY_VRAM);
-			upload_kernel<<<dim3(upload_tiles_x(c), upload_tiles_y(c)), 256, 0, stream>>>(c, d_vram);
+			upload_kernel<<<dim3((c.width + 31) / 32, (c.height + 7) / 8), 256, 0, stream>>>(c, d_vram);
 			launch_counter++;
 			CUDA_TRY(cudaGetLastError());
 			return PGS_OK;

@@ -3585,15 +3585,66 @@ __device__ __forceinline__ uint32_t read_pixel(const uint8_t *vram, uint32_t psm
 	return v32[a];
 }
 
-// Uploads go in tiles of 32 x 32 pixels from a multiple of 4 in the destination
-// on, a thread per four pixels of a row, which share one destination address
-// computation and, where they are aligned and all there, one payload load.
+// One pixel of a transfer.  A single transfer's launch is its latency (eight 16x16
+// uploads of one place, in turn: 20 us), so it takes the shortest code: four pixels
+// per thread, as in the batched uploads below, made them 25 to 29 us, and eight
+// 256x256 local copies 45 to 55 us instead of 35 to 41.
+__device__ __forceinline__ void upload_pixel(const CopyParams &C, uint8_t *vram, uint32_t x, uint32_t y)
+{
+	if (x >= C.width || y >= C.height)
+		return;
+	uint32_t eff_stride = C.dbw;
+	if (C.dpsm == PSMT4 || C.dpsm == PSMT8)
+		eff_stride &= ~1u;
+	if (x >= eff_stride * 64u)
+	{
+		Layout L = psm_layout(C.dpsm);
+		uint32_t last = (C.dsay + C.height - 1u) >> L.ph, cur = (C.dsay + y) >> L.ph;
+		if (last != cur)
+			return;
+	}
+	uint32_t dx = (x + C.dsax) & 2047u, dy = (y + C.dsay) & 2047u;
+	uint32_t data;
+	if (C.xdir == HOST_TO_LOCAL)
+	{
+		uint64_t sa = uint64_t(y) * C.width + x;
+		uint32_t b = psm_bits_per_pixel(C.dpsm);
+		uint64_t factor = (b == 32 || b == 24) ? 2 : (b == 16 ? 4 : (b == 8 ? 8 : 16));
+		uint64_t avail = b == 32 ? C.host_size / 4 : (b == 24 ? C.host_size / 3 : (b == 16 ? C.host_size / 2 : (b == 8 ? C.host_size : 2 * C.host_size)));
+		if (sa * factor < C.host_offset_qwords || sa >= avail)
+			return;
+		// The payload starts 256-byte aligned: a warp's 32 consecutive pixels
+		// read one contiguous span, with one load of the pixel's width each.
+		const uint8_t *h = C.host;
+		if (b == 24) data = uint32_t(h[3 * sa]) | (uint32_t(h[3 * sa + 1]) << 8) | (uint32_t(h[3 * sa + 2]) << 16);
+		else if (b == 16) data = reinterpret_cast<const uint16_t *>(h)[sa];
+		else if (b == 8) data = h[sa];
+		else if (b == 4) data = (uint32_t(h[sa >> 1]) >> ((sa & 1) * 4)) & 15u;
+		else data = reinterpret_cast<const uint32_t *>(h)[sa];
+	}
+	else
+	{
+		uint32_t sx = (x + C.ssax) & 2047u, sy = (y + C.ssay) & 2047u;
+		data = read_pixel(C.src_vram, C.spsm, swizzle_address(sx, sy, C.sbp, C.sbw, C.spsm));
+	}
+	write_pixel(vram, C.dpsm, swizzle_address(dx, dy, C.dbp, C.dbw, C.dpsm), data, C.invalidate_ss != 0);
+}
+
+__global__ void __launch_bounds__(256) upload_kernel(CopyParams C, uint8_t *vram)
+{
+	upload_pixel(C, vram, blockIdx.x * 32u + (threadIdx.x & 31u), blockIdx.y * 8u + (threadIdx.x >> 5));
+}
+
+// Batched uploads go in tiles of 32 x 32 pixels from a multiple of 4 in the
+// destination on, a thread per four pixels of a row, which share one destination
+// address computation and, where they are aligned and all there, one payload load.
 // Bound: issue of the address arithmetic (eight 256x256 PSMT8 textures with their
-// palettes: a pixel per thread 4.7 M warp instructions, so 1.8).
+// palettes: a pixel per thread 4.7 M warp instructions, so 1.8; a light frame that
+// uploads them 24.5 -> 22.9 us per replay).
 __host__ __device__ inline uint32_t upload_tiles_x(const CopyParams &C) { return ((C.dsax & 3u) + C.width + 31u) / 32u; }
 __host__ __device__ inline uint32_t upload_tiles_y(const CopyParams &C) { return (C.height + 31u) / 32u; }
 
-// Four pixels of the tile at (tx, ty).
+// Four pixels of the tile at (tx, ty) of a host->local upload.
 __device__ __forceinline__ void upload_quad(const CopyParams &C, uint8_t *vram, uint32_t tx, uint32_t ty)
 {
 	// Pixel k of the quad is column x0 + k of the rectangle (x0 may be negative).
@@ -3614,75 +3665,54 @@ __device__ __forceinline__ void upload_quad(const CopyParams &C, uint8_t *vram, 
 	const uint32_t dx = uint32_t(x0 + int32_t(C.dsax)) & 2047u, dy = (y + C.dsay) & 2047u;
 	uint32_t data[4];
 	uint32_t have = 0; // pixels to write
-	if (C.xdir == HOST_TO_LOCAL)
+	const uint32_t b = psm_bits_per_pixel(C.dpsm);
+	const uint32_t factor = (b == 32 || b == 24) ? 2 : (b == 16 ? 4 : (b == 8 ? 8 : 16));
+	const uint64_t avail = b == 32 ? C.host_size / 4 : (b == 24 ? C.host_size / 3 : (b == 16 ? C.host_size / 2 : (b == 8 ? C.host_size : 2 * C.host_size)));
+	const uint32_t row = y * C.width;
+	#pragma unroll
+	for (int k = 0; k < 4; k++)
 	{
-		const uint32_t b = psm_bits_per_pixel(C.dpsm);
-		const uint32_t factor = (b == 32 || b == 24) ? 2 : (b == 16 ? 4 : (b == 8 ? 8 : 16));
-		const uint64_t avail = b == 32 ? C.host_size / 4 : (b == 24 ? C.host_size / 3 : (b == 16 ? C.host_size / 2 : (b == 8 ? C.host_size : 2 * C.host_size)));
-		const uint32_t row = y * C.width;
-		#pragma unroll
-		for (int k = 0; k < 4; k++)
+		const int32_t x = x0 + k;
+		const uint64_t sa = uint64_t(row) + uint32_t(x);
+		if (x >= 0 && uint32_t(x) < limit && sa * factor >= C.host_offset_qwords && sa < avail)
+			have |= 1u << k;
+	}
+	if (!have)
+		return;
+	// The payload starts 256-byte aligned.
+	const uint8_t *h = C.host;
+	const uint32_t sa = row + uint32_t(x0); // of pixel 0, if it is there
+	if (have == 15u && !(sa & 3u) && (b == 32 || b == 16 || b == 8))
+	{
+		if (b == 32)
 		{
-			const int32_t x = x0 + k;
-			const uint64_t sa = uint64_t(row) + uint32_t(x);
-			if (x >= 0 && uint32_t(x) < limit && sa * factor >= C.host_offset_qwords && sa < avail)
-				have |= 1u << k;
+			const uint4 v = *reinterpret_cast<const uint4 *>(h + size_t(sa) * 4u);
+			data[0] = v.x; data[1] = v.y; data[2] = v.z; data[3] = v.w;
 		}
-		if (!have)
-			return;
-		// The payload starts 256-byte aligned.
-		const uint8_t *h = C.host;
-		const uint32_t sa = row + uint32_t(x0); // of pixel 0, if it is there
-		if (have == 15u && !(sa & 3u) && (b == 32 || b == 16 || b == 8))
+		else if (b == 16)
 		{
-			if (b == 32)
-			{
-				const uint4 v = *reinterpret_cast<const uint4 *>(h + size_t(sa) * 4u);
-				data[0] = v.x; data[1] = v.y; data[2] = v.z; data[3] = v.w;
-			}
-			else if (b == 16)
-			{
-				const uint2 v = *reinterpret_cast<const uint2 *>(h + size_t(sa) * 2u);
-				data[0] = v.x & 0xffffu; data[1] = v.x >> 16; data[2] = v.y & 0xffffu; data[3] = v.y >> 16;
-			}
-			else
-			{
-				const uint32_t v = *reinterpret_cast<const uint32_t *>(h + sa);
-				data[0] = v & 0xffu; data[1] = (v >> 8) & 0xffu; data[2] = (v >> 16) & 0xffu; data[3] = v >> 24;
-			}
+			const uint2 v = *reinterpret_cast<const uint2 *>(h + size_t(sa) * 2u);
+			data[0] = v.x & 0xffffu; data[1] = v.x >> 16; data[2] = v.y & 0xffffu; data[3] = v.y >> 16;
 		}
 		else
 		{
-			#pragma unroll
-			for (int k = 0; k < 4; k++)
-			{
-				if (!((have >> k) & 1u))
-					continue;
-				const size_t p = size_t(row) + uint32_t(x0 + k);
-				if (b == 24) data[k] = uint32_t(h[3 * p]) | (uint32_t(h[3 * p + 1]) << 8) | (uint32_t(h[3 * p + 2]) << 16);
-				else if (b == 16) data[k] = reinterpret_cast<const uint16_t *>(h)[p];
-				else if (b == 8) data[k] = h[p];
-				else if (b == 4) data[k] = (uint32_t(h[p >> 1]) >> ((p & 1) * 4)) & 15u;
-				else data[k] = reinterpret_cast<const uint32_t *>(h)[p];
-			}
+			const uint32_t v = *reinterpret_cast<const uint32_t *>(h + sa);
+			data[0] = v & 0xffu; data[1] = (v >> 8) & 0xffu; data[2] = (v >> 16) & 0xffu; data[3] = v >> 24;
 		}
 	}
 	else
 	{
-		// One address for all four where the source is as aligned as the destination.
-		const uint32_t sy = (y + C.ssay) & 2047u;
-		const bool aligned = !((C.ssax ^ C.dsax) & 3u);
-		const uint32_t sa = swizzle_address(uint32_t(x0 + int32_t(C.ssax)) & 2047u, sy, C.sbp, C.sbw, C.spsm);
 		#pragma unroll
 		for (int k = 0; k < 4; k++)
 		{
-			const int32_t x = x0 + k;
-			if (x < 0 || uint32_t(x) >= limit)
+			if (!((have >> k) & 1u))
 				continue;
-			const uint32_t s = aligned ? sa + quad_offset(C.spsm, uint32_t(k))
-			                           : swizzle_address((uint32_t(x) + C.ssax) & 2047u, sy, C.sbp, C.sbw, C.spsm);
-			data[k] = read_pixel(C.src_vram, C.spsm, s);
-			have |= 1u << k;
+			const size_t p = size_t(row) + uint32_t(x0 + k);
+			if (b == 24) data[k] = uint32_t(h[3 * p]) | (uint32_t(h[3 * p + 1]) << 8) | (uint32_t(h[3 * p + 2]) << 16);
+			else if (b == 16) data[k] = reinterpret_cast<const uint16_t *>(h)[p];
+			else if (b == 8) data[k] = h[p];
+			else if (b == 4) data[k] = (uint32_t(h[p >> 1]) >> ((p & 1) * 4)) & 15u;
+			else data[k] = reinterpret_cast<const uint32_t *>(h)[p];
 		}
 	}
 	const uint32_t a = swizzle_address(dx, dy, C.dbp, C.dbw, C.dpsm);
@@ -3690,11 +3720,6 @@ __device__ __forceinline__ void upload_quad(const CopyParams &C, uint8_t *vram, 
 	for (int k = 0; k < 4; k++)
 		if ((have >> k) & 1u)
 			write_pixel(vram, C.dpsm, a + quad_offset(C.dpsm, uint32_t(k)), data[k], C.invalidate_ss != 0);
-}
-
-__global__ void __launch_bounds__(256) upload_kernel(CopyParams C, uint8_t *vram)
-{
-	upload_quad(C, vram, blockIdx.x, blockIdx.y);
 }
 
 // Consecutive host->local uploads whose destination blocks do not overlap, in
