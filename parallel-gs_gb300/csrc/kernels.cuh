@@ -2098,137 +2098,82 @@ __device__ __forceinline__ void sample_offset(uint32_t s, uint32_t xl, uint32_t 
 
 // Processes one primitive for the calling warp: coverage, early depth,
 // deferred-shading bookkeeping (ubershader.comp:1694-1812).  Warp-uniform.
-// The 8x8 bins already hold only primitives that intersect the sub-tile
-// (primitive_intersects_tile); a second test against each warp's smaller
-// rectangle costs more than the coverage test it would skip, so coverage
-// alone decides.
-template <bool SS, bool MIP>
-__device__ __forceinline__ void process_primitive_with(const ShadeCtx &C, uint32_t pi, const PrimSetup &s, uint32_t st,
-                                                       SampleState &S, uint32_t &covered)
+// A primitive that is not opaque (warp-uniform: a state bit) is shaded right
+// away rather than left pending.  The result is the same as shading it at the
+// next flush: leaving it pending only saves work when a later opaque primitive
+// covers the sample, which blended primitives seldom meet, and shading now keeps
+// every lane of the call on the same primitive.  What was pending is shaded first
+// wherever this primitive covers a sample that has a pending one.  An opaque one
+// replaces what was pending and writes its depth, so a pending primitive never
+// has a depth test or write left to do.  With `flush` there is no primitive and
+// all that is pending is shaded.
+// With mip levels or layered textures the shading code is long: a copy of it for
+// each call (five) had the warps wait 15 cycles per issue for instructions, so one
+// call in a rolled loop serves both shadings and the flush (25,000 small mip-mapped
+// triangles at 8x 652 -> 341 us, at 16x 1126 -> 572).  Without, two copies here and
+// one behind the walk are faster: 10,000 mixed AA1 primitives at 4x 291 us, rolled 312.
+template <bool MIP>
+__device__ __forceinline__ void process_primitive(const ShadeCtx &C, uint32_t pi, bool flush, SampleState &S, uint32_t &covered)
 {
-	bool opaque, any_cov;
-	Request q = shade_early<MIP>(C, s, pi, st, S, opaque, any_cov);
-	if (!any_cov)
-		return;
-	// A primitive that is not opaque (warp-uniform: a state bit) is shaded
-	// right away rather than left pending.  The result is the same as shading
-	// it at the next flush: leaving it pending only saves work when a later
-	// opaque primitive covers the sample, which blended primitives seldom
-	// meet, and shading now keeps every lane of the call on the same
-	// primitive.  What was pending is shaded first wherever this primitive
-	// covers a sample that has a pending one.  The super-sampled variants take
-	// this path on its own; the single-sampled one keeps the shared path below
-	// (measured: the separate path speeds the first up and slows the second).
-	if (SS && !opaque)
+	const PassParams &P = *C.P;
+	const unsigned full = 0xffffffffu;
+	Request q;
+	q.coverage = 0;
+	bool before = S.pending.coverage > 0;
+	if (!flush)
 	{
-		if (q.coverage > 0)
+		const PrimSetup s = P.setup[pi];
+		const uint32_t st = P.prims[pi].state;
+		bool opaque, any_cov;
+		q = shade_early<MIP>(C, s, pi, st, S, opaque, any_cov);
+		if (!any_cov)
+			return;
+		covered += q.coverage > 0 ? 1u : 0u;
+		if (q.z_test)
 		{
-			covered++;
-			if (q.z_test && !S.pending.z_write)
-			{
-				const bool zp = ((st >> STATE_BIT_Z_TEST_GREATER) & 1) ? q.z > S.depth : q.z >= S.depth;
-				if (!zp)
-				{
-					q.coverage = 0;
-					q.z_write = false;
-				}
-				q.z_test = false;
-			}
+			if (!(((st >> STATE_BIT_Z_TEST_GREATER) & 1) ? q.z > S.depth : q.z >= S.depth))
+				q.coverage = 0;
+			q.z_test = false;
 		}
-		if (__any_sync(0xffffffffu, q.coverage > 0 && S.pending.coverage > 0))
-		{
-			if (S.pending.coverage > 0)
-				shade_resolve<MIP, true>(C, S, S.pending_prim, S.pending);
-			S.pending.coverage = 0;
-			S.pending.z_write = false;
-		}
-		if (__any_sync(0xffffffffu, q.coverage > 0))
+		if (opaque)
 		{
 			if (q.coverage > 0)
 			{
-				S.pending = q;
-				S.pending_prim = pi;
-				shade_resolve<MIP, true>(C, S, S.pending_prim, S.pending);
-				S.pending.coverage = 0;
-				S.pending.z_write = false;
-			}
-		}
-		return;
-	}
-	if (q.coverage > 0)
-	{
-		covered++;
-		if (q.z_test && !S.pending.z_write)
-		{
-			q.z_test = false;
-			bool zp = ((st >> STATE_BIT_Z_TEST_GREATER) & 1) ? q.z > S.depth : q.z >= S.depth;
-			if (zp)
-			{
-				if (q.z_write && opaque)
+				if (q.z_write)
 				{
-					q.z_write = false;
 					S.depth = q.z;
 					S.depth_dirty = true;
 				}
+				S.pending.coverage = q.coverage;
+				S.pending.i = q.i;
+				S.pending.j = q.j;
+				S.pending_prim = pi;
 			}
-			else
-			{
-				q.coverage = 0;
-				q.z_write = false;
-			}
+			return;
 		}
-		else if (q.z_write && !q.z_test && opaque)
-		{
-			q.z_write = false;
-			S.pending.z_write = false;
-			S.depth = q.z;
-			S.depth_dirty = true;
-		}
-		if ((q.z_test || !q.z_write) && S.pending.z_write)
-			opaque = false;
+		if (!__any_sync(full, q.coverage > 0))
+			return;
+		if (!__any_sync(full, q.coverage > 0 && before))
+			before = false;
 	}
-	bool need_flush = false;
-	if (q.coverage > 0)
+	#pragma unroll (MIP ? 1 : 2)
+	for (uint32_t step = __any_sync(full, before) ? 0u : 1u; step < (flush ? 1u : 2u); step++)
 	{
-		need_flush = !opaque && S.pending.coverage > 0;
-		if (!need_flush)
+		Request r = q;
+		uint32_t rp = pi;
+		if (!step)
 		{
-			S.pending = q;
-			S.pending_prim = pi;
-			q.coverage = 0;
-		}
-	}
-	if (__any_sync(0xffffffffu, need_flush))
-	{
-		if (S.pending.coverage > 0)
-			shade_resolve<MIP, true>(C, S, S.pending_prim, S.pending);
-		S.pending.coverage = 0;
-		S.pending.z_write = false;
-		if (q.coverage > 0)
-		{
-			S.pending = q;
-			S.pending_prim = pi;
-		}
-	}
-	// The shared path shades a primitive that is not opaque at once too.
-	if (!((st >> STATE_BIT_OPAQUE) & 1u) &&
-	    __any_sync(0xffffffffu, S.pending.coverage > 0 && S.pending_prim == pi))
-	{
-		if (S.pending.coverage > 0 && S.pending_prim == pi)
-		{
-			shade_resolve<MIP, true>(C, S, S.pending_prim, S.pending);
+			r.coverage = before ? S.pending.coverage : 0;
+			r.i = S.pending.i;
+			r.j = S.pending.j;
+			r.z_write = false;
+			rp = S.pending_prim;
 			S.pending.coverage = 0;
-			S.pending.z_write = false;
 		}
+		r.z_test = false;
+		if (r.coverage > 0)
+			shade_resolve<MIP, true>(C, S, rp, r);
 	}
-}
-
-template <bool SS, bool MIP>
-__device__ __forceinline__ void process_primitive(const ShadeCtx &C, uint32_t pi, SampleState &S, uint32_t &covered)
-{
-	const PassParams &P = *C.P;
-	const PrimSetup s = P.setup[pi];
-	process_primitive_with<SS, MIP>(C, pi, s, P.prims[pi].state, S, covered);
 }
 
 // ---------------------------------------------------------------------------
@@ -2799,7 +2744,7 @@ __device__ __forceinline__ void walk_list(const ShadeCtx &C, const DevInstance &
 					                   S, covered);
 			}
 			else
-			for (uint32_t kb = 0; kb < n; kb += 32u)
+			for (uint32_t kb = 0; kb < n || (last_round && kb == 0); kb += 32u)
 			{
 				const uint32_t k = kb + lane;
 				uint32_t pi = 0;
@@ -2810,11 +2755,16 @@ __device__ __forceinline__ void walk_list(const ShadeCtx &C, const DevInstance &
 					hit = may_cover(P.setup[pi], P.prims[pi].state, rect, C.dim);
 				}
 				uint32_t bits = __ballot_sync(full, hit);
-				while (bits)
+				// Behind the sub-tile's last primitive, what is pending.
+				const bool last = MIP && last_round && kb + 32u >= n;
+				while (bits || last)
 				{
-					const int b = __ffs(bits) - 1;
+					const bool flush = !bits;
+					const int b = flush ? 0 : __ffs(bits) - 1;
 					bits &= bits - 1u;
-					process_primitive<SS, MIP>(C, __shfl_sync(full, pi, b), S, covered);
+					process_primitive<MIP>(C, __shfl_sync(full, pi, b), flush, S, covered);
+					if (flush)
+						break;
 				}
 			}
 		}
@@ -2954,8 +2904,8 @@ __device__ __forceinline__ void shade_part(const PassParams &P, const DevInstanc
 	uint32_t covered = 0;
 	walk_list<NS, SS, AA, MIP, RELOAD, T, CAP>(C, I, G, mask, chunk, written, list, t, S, covered);
 
-	// walk_batch leaves nothing pending.
-	if (AA && S.pending.coverage > 0)
+	// The other walks shade what is pending behind their last primitive.
+	if (AA && !MIP && S.pending.coverage > 0)
 		shade_resolve<MIP, AA>(C, S, S.pending_prim, S.pending);
 
 	// Covered-sample counter: one atomic per warp.
