@@ -251,6 +251,7 @@ constexpr size_t CLUT_BYTES = size_t(PGS_CLUT_INSTANCES) * PGS_CLUT_SIZE_BYTES;
 struct CudaBackend
 {
 	int device = 0;
+	int sm_count = 0;
 	cudaStream_t stream = nullptr;
 	uint32_t max_planes = 1;
 	uint32_t num_planes = 1;
@@ -434,6 +435,7 @@ struct CudaBackend
 		if (device < 0 || device >= count)
 			return PGS_ERROR_INVALID_ARGUMENT;
 		CUDA_TRY(cudaSetDevice(device));
+		CUDA_TRY(cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, device));
 		CUDA_TRY(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
 		uint32_t ms = opt ? std::min<uint32_t>(opt->max_samples_log2, 4) : 4;
 		max_planes = ms ? 2u + (1u << ms) : 1u;
@@ -1081,6 +1083,9 @@ struct CudaBackend
 		return depth;
 	}
 
+	// Shading CTAs of 256 threads that the GPU holds at a time.
+	uint32_t shade_slots() const { return uint32_t(sm_count) * PGS_SHADE_MIN_BLOCKS(PGS_SHADE_CTA_NS); }
+
 	// Shading launches: the super-sampled variant for tiles that need it, then
 	// the single-sampled variant (ubershader.comp dispatched twice,
 	// gs/gs_renderer.cpp:2395-2415).
@@ -1090,12 +1095,14 @@ struct CudaBackend
 	{
 		if (I.rate_y_log2 != 0)
 		{
+			// Behind the sub-tiles' CTAs those for the parts of split ones, as many as fit the GPU.
+			const uint32_t more = I.split_count ? std::min(shade_slots(), grid << (ns_log2 - 2u)) : 0u;
 			switch (ns_log2)
 			{
 			case 1: shade_kernel<2, true, AA, MIP><<<grid, ShadeCta<2>::THREADS, 0, stream>>>(P, I, masks, d_flags); break;
 			case 2: shade_kernel<4, true, AA, MIP><<<grid, ShadeCta<4>::THREADS, 0, stream>>>(P, I, masks, d_flags); break;
-			case 3: shade_kernel<8, true, AA, MIP><<<grid, ShadeCta<8>::THREADS, 0, stream>>>(P, I, masks, d_flags); break;
-			default: shade_kernel<16, true, AA, MIP><<<grid, ShadeCta<16>::THREADS, 0, stream>>>(P, I, masks, d_flags); break;
+			case 3: shade_kernel<8, true, AA, MIP><<<grid + more, ShadeCta<8>::THREADS, 0, stream>>>(P, I, masks, d_flags); break;
+			default: shade_kernel<16, true, AA, MIP><<<grid + more, ShadeCta<16>::THREADS, 0, stream>>>(P, I, masks, d_flags); break;
 			}
 			launch_counter++;
 		}
@@ -1147,6 +1154,15 @@ struct CudaBackend
 		// Super-sampled shading touches planes 1 .. 1 + 2^ns_log2.
 		if (I.rate_y_log2 != 0 && 2u + (1u << ns_log2) > num_planes)
 			return PGS_ERROR_INVALID_ARGUMENT;
+		// 8x and 16x: coarse tiles from this many primitives on have their sub-tiles
+		// split (ShadeCta).  Blended triangles in one sub-tile at 16x in turn and in
+		// CTAs of 1024 threads, which hold it whole: 300 0.39 and 0.67 ms, 2,000 2.41
+		// and 1.99; AA1 triangles 300 0.55 and 0.67, 2,000 3.15 and 1.88.  Not where
+		// tiles like it, if the pass consists of them, fill the GPU anyway: 20,000
+		// sprites all over the frame at 16x 676 us, with a CTA per part 695.
+		const uint32_t from = p.has_aa1 || p.has_mipmap || p.has_ss_textures ? 256u : 1024u;
+		if (ns_log2 > 2 && count >= from)
+			I.split_count = std::max(from, uint32_t((uint64_t(count) << (2u * (p.tile_size_log2 - 3u))) / shade_slots()));
 		size_t mask_words = subs * I.mask_words;
 		// Sub-tile masks and the coarse tiles' flags, cleared together.
 		int r = ensure_masks(mask_words + tiles);

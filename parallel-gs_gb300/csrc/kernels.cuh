@@ -70,6 +70,7 @@ struct DevInstance
 	int32_t snap_mask_y;          // raster snap of rows: half the sample pitch when field rendering
 	uint32_t force_ss;            // field rendering: every covered tile super-sampled
 	uint32_t blend_demote;        // primitives per coarse tile that demote a blended tile, 0 = off
+	uint32_t split_count;         // primitives per coarse tile that split its sub-tiles (split_tile), 0 = never
 };
 
 // Linear RGBA8 image decoded from swizzled VRAM + CLUT for one mip level of
@@ -207,7 +208,8 @@ constexpr uint32_t TILE_NONEMPTY = 1u << 0;
 constexpr uint32_t TILE_REQ_SS = 1u << 1;
 constexpr uint32_t TILE_REQ_SS_ZW = 1u << 2;
 constexpr uint32_t TILE_HAS_ZW = 1u << 3;
-// Primitives binned to the tile, counted from this bit when blend demotion is on.
+// Primitives binned to the tile, counted from this bit for blend demotion, or by
+// every eighth primitive for splitting.
 constexpr uint32_t TILE_COUNT_SHIFT = 8;
 
 constexpr uint32_t ERROR_FLAG_TILE_OVERFLOW = 1u << 0;
@@ -1097,8 +1099,11 @@ __global__ void __launch_bounds__(32 * BIN_GROUP_WARPS) bin_kernel(PassParams P,
 
 	auto mark_tile = [&](const BinItem &it, uint32_t tile) {
 		atomicOr(&tile_flags[tile], it.flags);
+		// All of them counted for splitting as well take a launch of 20,000 primitives from 8.5 to 13 us.
 		if (I.blend_demote)
 			atomicAdd(&tile_flags[tile], 1u << TILE_COUNT_SHIFT);
+		else if (I.split_count && !(it.local & 7u))
+			atomicAdd(&tile_flags[tile], 8u << TILE_COUNT_SHIFT);
 	};
 	if (ts > 3)
 		deal_tiles(items, n, ts, [&](const BinItem &it, int32_t tx, int32_t ty) {
@@ -2586,6 +2591,11 @@ __device__ __forceinline__ void walk_batch(const ShadeCtx &C, const uint32_t *id
 // of them per SM, waiting for each other at every barrier; a CTA per part expands
 // the list again and starts more CTAs (feedback frame of 100,000 primitives at 8x
 // 2.48 ms whole, 1.93 a CTA per part, 1.72 so; at 16x 5.07, 3.51, 2.74).
+// A long list is the launch's critical path, though, and the parts in turn make it
+// as many times longer, so the sub-tiles of coarse tiles with many primitives are
+// split: CTAs behind those of the sub-tiles take their parts (2,000 blended
+// triangles in one sub-tile at 16x 2.41 -> 0.77 ms, 36,000 AA1 triangles within
+// 64x64 pixels 2.13 -> 0.67).  Which tiles: run_instance.
 template <int NS>
 struct ShadeCta
 {
@@ -2776,14 +2786,10 @@ __device__ __forceinline__ void walk_list(const ShadeCtx &C, const DevInstance &
 	}
 }
 
-// Coarse-tile state of sub-tile `sub`: 0 = empty, 1 = single-sampled,
+// State of a coarse tile with these flags: 0 = empty, 1 = single-sampled,
 // 2 = super-sampled (binning.comp:272-311 decision).
-__device__ __forceinline__ uint32_t subtile_mode(const PassParams &P, const DevInstance &I, const uint32_t *tile_flags,
-                                                 uint32_t sub)
+__device__ __forceinline__ uint32_t tile_mode(const DevInstance &I, uint32_t flags)
 {
-	const uint32_t gx = sub % I.sub_w, gy = sub / I.sub_w;
-	const uint32_t sh = P.tile_size_log2 - 3u;
-	const uint32_t flags = tile_flags[(gy >> sh) * I.tiles_w + (gx >> sh)];
 	if (!(flags & TILE_NONEMPTY))
 		return 0;
 	bool req = I.force_ss || (flags & TILE_REQ_SS);
@@ -2791,6 +2797,61 @@ __device__ __forceinline__ uint32_t subtile_mode(const PassParams &P, const DevI
 		req = false;
 	req = req || ((flags & TILE_REQ_SS_ZW) && (flags & TILE_HAS_ZW));
 	return (I.rate_y_log2 != 0 && req) ? 2u : 1u;
+}
+
+// Flags of the coarse tile of sub-tile `sub`.
+__device__ __forceinline__ uint32_t subtile_flags(const PassParams &P, const DevInstance &I, const uint32_t *tile_flags,
+                                                  uint32_t sub)
+{
+	const uint32_t gx = sub % I.sub_w, gy = sub / I.sub_w;
+	const uint32_t sh = P.tile_size_log2 - 3u;
+	return tile_flags[(gy >> sh) * I.tiles_w + (gx >> sh)];
+}
+
+// Whether the parts of the sub-tiles of a coarse tile go to CTAs of their own
+// (ShadeCta).  Which CTA shades a part changes no result.
+__device__ __forceinline__ bool split_tile(const DevInstance &I, uint32_t flags)
+{
+	return I.split_count && (flags >> TILE_COUNT_SHIFT) >= I.split_count;
+}
+
+// Part number `item` of all parts of the sub-tiles of split super-sampled tiles:
+// its sub-tile and part, or false behind the last.  All threads of the group.
+template <uint32_t PARTS, uint32_t T, uint32_t CAP>
+__device__ __forceinline__ bool split_part(const PassParams &P, const DevInstance &I, const uint32_t *tile_flags, uint32_t item,
+                                           const ShadeGroup<T> &G, ListShared<T, CAP> &list, uint32_t &sub, uint32_t &part)
+{
+	const uint32_t sh = P.tile_size_log2 - 3u, per_tile = PARTS << (2u * sh);
+	const uint32_t want = item / per_tile, k = item % per_tile; // tile by rank, part in it
+	const uint32_t lane = G.thread() & 31u, warp = G.thread() >> 5, tiles = I.tiles_w * I.tiles_h;
+	uint32_t seen = 0;
+	for (uint32_t base = 0; base < tiles; base += T)
+	{
+		const uint32_t tile = base + G.thread(), flags = tile < tiles ? tile_flags[tile] : 0u;
+		const bool split = tile_mode(I, flags) == 2u && split_tile(I, flags);
+		const uint32_t m = __ballot_sync(0xffffffffu, split);
+		if (lane == 0)
+			list.count[warp] = uint32_t(__popc(m));
+		G.sync();
+		uint32_t rank = seen + uint32_t(__popc(m & ((1u << lane) - 1u)));
+		for (uint32_t w = 0; w < T / 32u; w++)
+		{
+			const uint32_t c = list.count[w];
+			rank += w < warp ? c : 0u;
+			seen += c;
+		}
+		if (split && rank == want)
+			list.ids[0] = tile;
+		G.sync();
+		if (want < seen)
+		{
+			const uint32_t t = list.ids[0], in = k / PARTS;
+			sub = ((t / I.tiles_w << sh) + (in >> sh)) * I.sub_w + (t % I.tiles_w << sh) + (in & ((1u << sh) - 1u));
+			part = k % PARTS;
+			return true;
+		}
+	}
+	return false;
 }
 
 // Samples t of the sub-tile at (sub_x, sub_y), one per thread of the group.
@@ -3108,15 +3169,29 @@ template <int NS, bool SS, bool AA, bool MIP>
 __global__ void __launch_bounds__(ShadeCta<NS>::THREADS, PGS_SHADE_MIN_BLOCKS(NS)) shade_kernel(PassParams P, DevInstance I, const uint32_t *sub_masks,
                                                         const uint32_t *tile_flags)
 {
-	constexpr uint32_t T = ShadeCta<NS>::THREADS;
+	constexpr uint32_t T = ShadeCta<NS>::THREADS, PARTS = ShadeCta<NS>::PARTS;
 	__shared__ ListShared<T, SHADE_LIST_CAP> list;
-	const uint32_t sub = blockIdx.x;
-	if (sub >= I.sub_w * I.sub_h)
+	const ShadeGroup<T> G{ 0u };
+	const uint32_t subs = I.sub_w * I.sub_h;
+	uint32_t sub = blockIdx.x;
+	// The usual case comes first: behind the other, each launch took 3 us longer.
+	if (sub < subs)
+	{
+		const uint32_t flags = subtile_flags(P, I, tile_flags, sub);
+		if (tile_mode(I, flags) == (SS ? 2u : 1u) && !(PARTS > 1 && split_tile(I, flags)))
+			shade_subtile<NS, SS, AA, MIP, PARTS, T, SHADE_LIST_CAP>(P, I, G, sub_masks, sub, threadIdx.x, list);
 		return;
-	if (subtile_mode(P, I, tile_flags, sub) != (SS ? 2u : 1u))
-		return;
-	shade_subtile<NS, SS, AA, MIP, ShadeCta<NS>::PARTS, T, SHADE_LIST_CAP>(P, I, ShadeGroup<T>{ 0u }, sub_masks, sub, threadIdx.x,
-	                                                                       list);
+	}
+	if constexpr (PARTS > 1)
+	{
+		// Parts of split sub-tiles, one after another.
+		uint32_t part;
+		for (uint32_t item = sub - subs; split_part<PARTS>(P, I, tile_flags, item, G, list, sub, part); item += gridDim.x - subs)
+		{
+			shade_subtile<NS, SS, AA, MIP, 1, T, SHADE_LIST_CAP>(P, I, G, sub_masks, sub, threadIdx.x + part * T, list);
+			__syncthreads();
+		}
+	}
 }
 
 // ---------------------------------------------------------------------------
@@ -3204,7 +3279,7 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) batch_shade_kernel(const 
 		}
 		const uint32_t sample = (unit - it.unit_base) * BLOCK + threadIdx.x;
 		const uint32_t sub = sample >> (6u + it.ns_log2), t = sample & ((64u << it.ns_log2) - 1u);
-		const uint32_t mode = sub < I.sub_w * I.sub_h ? subtile_mode(P, I, it.flags, sub) : 0u;
+		const uint32_t mode = sub < I.sub_w * I.sub_h ? tile_mode(I, subtile_flags(P, I, it.flags, sub)) : 0u;
 		const uint32_t ns_log2 = mode == 2 ? it.ns_log2 : 0u;
 		// A group's barrier and list are those of its first 64 threads.
 		if (mode && t < (64u << ns_log2))
