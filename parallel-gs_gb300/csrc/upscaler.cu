@@ -772,7 +772,7 @@ __global__ void __launch_bounds__(128) umma_probe_kernel(uint32_t mode, float *o
 // forward half of training).  Persistent CTAs own tiles of 16 rows x 8 columns
 // = 128 output pixels.  Warp-specialised pipeline:
 //  - warp 5, one lane: TMA loads of each tile's 18 x 10 x 32 input window (zero
-//    fill outside the image, 64-byte swizzle), five stages.  It is not the lane
+//    fill outside the image, 64-byte swizzle), three or five stages.  It is not the lane
 //    that issues the MMAs: refilling a stage waits for the MMAs that read it, and
 //    one lane for both let the tensor cores run dry at every tile;
 //  - warp 0, one lane: 9 taps x 2 K-steps of tcgen05.mma (M 128, N 32, K 16)
@@ -797,20 +797,27 @@ namespace tc
 {
 constexpr int ROWS = 16, COLS = 8;
 constexpr int WIN_ROWS = ROWS + 2, WIN_COLS = COLS + 2;
-constexpr int STAGES = 5, ACCS = 4;
+constexpr int ACCS = 4;
+// Stages of input.  With five, two CTAs fill an SM's shared memory; with three, the
+// next layer's CTAs (inference, programmatic dependent launch) get in beside them and
+// are set up by the time this layer ends, which is what counts while a frame has few
+// tiles.  Network on a frame of 192x256 (384 tiles) 42.2 us with five, 33.0 with
+// three, 224x320 (560) 44.7 and 35.2, 256x384 (768) 48.4 and 46.4, 320x384 (960) 52.0
+// and 51.1; then the five gain: 384x512 (1536) 63.2 and 66.6, 1080x1920 395 and 440.
+constexpr int STAGES_MANY = 5, STAGES_FEW = 3, FEW_TILES = 6; // per SM
 constexpr uint32_t ROW_BYTES = WIN_COLS * 64;               // 640
 constexpr uint32_t WIN_BYTES = WIN_ROWS * ROW_BYTES;        // 11520
 constexpr uint32_t STAGE_BYTES = 12288;                     // a window from a 1 KiB boundary
 constexpr uint32_t W_BYTES = 9 * 32 * 64;                   // 18432
 constexpr uint32_t OUT_BYTES = 32 * 64;                     // one warp's 8 x 4 pixels
 constexpr int OUT_BUFS = 2;
-constexpr uint32_t SMEM_BYTES = 1024 + STAGES * STAGE_BYTES + W_BYTES + 4 * OUT_BUFS * OUT_BYTES;
+constexpr uint32_t smem_bytes(int stages) { return 1024 + stages * STAGE_BYTES + W_BYTES + 4 * OUT_BUFS * OUT_BYTES; }
 constexpr int THREADS = 192;
 }
 
 // EPI_RELU writes relu(acc + bias); EPI_MASK (the data gradient of a 32 -> 32
 // layer through the ReLU before it) writes acc where mask > 0, else 0.
-template <int EPI>
+template <int EPI, int STAGES>
 __global__ void __launch_bounds__(tc::THREADS, 2) conv32_tc_kernel(const __grid_constant__ CUtensorMap tmap,
                                                                     const __grid_constant__ CUtensorMap out_map,
                                                                     const __nv_bfloat16 *wt, const float *bias,
@@ -820,8 +827,8 @@ __global__ void __launch_bounds__(tc::THREADS, 2) conv32_tc_kernel(const __grid_
 	using namespace pgs_umma;
 	extern __shared__ uint8_t smem_dyn[];
 	uint8_t *base = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~uintptr_t(1023));
-	uint8_t *sw = base + tc::STAGES * tc::STAGE_BYTES, *sout = sw + tc::W_BYTES;
-	__shared__ uint64_t full_bar[tc::STAGES], empty_bar[tc::STAGES], acc_full[tc::ACCS], acc_empty[tc::ACCS];
+	uint8_t *sw = base + STAGES * tc::STAGE_BYTES, *sout = sw + tc::W_BYTES;
+	__shared__ uint64_t full_bar[STAGES], empty_bar[STAGES], acc_full[tc::ACCS], acc_empty[tc::ACCS];
 	__shared__ uint32_t tmem_slot;
 	__shared__ __align__(16) float s_bias[32];
 	__shared__ volatile uint32_t s_abort;
@@ -844,7 +851,7 @@ __global__ void __launch_bounds__(tc::THREADS, 2) conv32_tc_kernel(const __grid_
 		tmem_alloc(&tmem_slot, tc::ACCS * 32);
 	if (tid == 0)
 	{
-		for (int s = 0; s < tc::STAGES; s++)
+		for (int s = 0; s < STAGES; s++)
 		{
 			mbar_init(&full_bar[s], 1);
 			mbar_init(&empty_bar[s], 1);
@@ -883,8 +890,8 @@ __global__ void __launch_bounds__(tc::THREADS, 2) conv32_tc_kernel(const __grid_
 			const uint64_t bd = smem_desc(smem_addr(sw), 16, 512, LAYOUT_SWIZZLE_64B);
 			for (int i = 0; i < mine && !s_abort; i++)
 			{
-				const int s = i % tc::STAGES, a = i % tc::ACCS;
-				if (!mbar_wait_or_abort(&full_bar[s], (i / tc::STAGES) & 1, &s_abort) ||
+				const int s = i % STAGES, a = i % tc::ACCS;
+				if (!mbar_wait_or_abort(&full_bar[s], (i / STAGES) & 1, &s_abort) ||
 				    (i >= tc::ACCS && !mbar_wait_or_abort(&acc_empty[a], ((i / tc::ACCS) - 1) & 1, &s_abort)))
 				{
 					atomicOr(err, 2u);
@@ -919,8 +926,8 @@ __global__ void __launch_bounds__(tc::THREADS, 2) conv32_tc_kernel(const __grid_
 			int i = 0;
 			for (; i < mine && !s_abort; i++)
 			{
-				const int s = i % tc::STAGES;
-				if (i >= tc::STAGES && !mbar_wait_or_abort(&empty_bar[s], ((i / tc::STAGES) - 1) & 1, &s_abort))
+				const int s = i % STAGES;
+				if (i >= STAGES && !mbar_wait_or_abort(&empty_bar[s], ((i / STAGES) - 1) & 1, &s_abort))
 				{
 					atomicOr(err, 1u);
 					s_abort = 1;
@@ -933,8 +940,8 @@ __global__ void __launch_bounds__(tc::THREADS, 2) conv32_tc_kernel(const __grid_
 			}
 			// Given up: the copies in flight still have to land.
 			if (s_abort)
-				for (int k = (i > tc::STAGES ? i - tc::STAGES : 0); k < i; k++)
-					mbar_wait_limit(&full_bar[k % tc::STAGES], (k / tc::STAGES) & 1, 1u << 20);
+				for (int k = (i > STAGES ? i - STAGES : 0); k < i; k++)
+					mbar_wait_limit(&full_bar[k % STAGES], (k / STAGES) & 1, 1u << 20);
 		}
 		__syncwarp();
 	}
@@ -1153,10 +1160,11 @@ struct Upscaler
 		UP_TRY(cudaMalloc(&d_loss, sizeof(double)));
 		UP_TRY(cudaMalloc(&d_err, sizeof(uint32_t)));
 		UP_TRY(cudaMemset(d_err, 0, sizeof(uint32_t)));
-		UP_TRY(cudaFuncSetAttribute(conv32_tc_kernel<EPI_RELU>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-		                            int(tc::SMEM_BYTES)));
-		UP_TRY(cudaFuncSetAttribute(conv32_tc_kernel<EPI_MASK>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-		                            int(tc::SMEM_BYTES)));
+		const int few = int(tc::smem_bytes(tc::STAGES_FEW)), many = int(tc::smem_bytes(tc::STAGES_MANY));
+		const cudaFuncAttribute attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
+		UP_TRY(cudaFuncSetAttribute(conv32_tc_kernel<EPI_RELU, tc::STAGES_FEW>, attr, few));
+		UP_TRY(cudaFuncSetAttribute(conv32_tc_kernel<EPI_RELU, tc::STAGES_MANY>, attr, many));
+		UP_TRY(cudaFuncSetAttribute(conv32_tc_kernel<EPI_MASK, tc::STAGES_MANY>, attr, many));
 		return PGS_OK;
 	}
 
@@ -1272,8 +1280,12 @@ struct Upscaler
 			return r;
 		int tiles = ((a.w + tc::COLS - 1) / tc::COLS) * ((a.h + tc::ROWS - 1) / tc::ROWS) * a.n;
 		int grid = std::min(tiles, sm_count * use_tc);
-		return launch(conv32_tc_kernel<EPI>, dim3(grid), dim3(tc::THREADS), tc::SMEM_BYTES, pdl, in, out, a.wt, a.bias,
-		              a.mask, a.n, a.h, a.w, d_err);
+		if constexpr (EPI == EPI_RELU)
+			if (pdl && tiles <= tc::FEW_TILES * sm_count)
+				return launch(conv32_tc_kernel<EPI, tc::STAGES_FEW>, dim3(grid), dim3(tc::THREADS),
+				              tc::smem_bytes(tc::STAGES_FEW), pdl, in, out, a.wt, a.bias, a.mask, a.n, a.h, a.w, d_err);
+		return launch(conv32_tc_kernel<EPI, tc::STAGES_MANY>, dim3(grid), dim3(tc::THREADS), tc::smem_bytes(tc::STAGES_MANY),
+		              pdl, in, out, a.wt, a.bias, a.mask, a.n, a.h, a.w, d_err);
 	}
 
 	template <int CIN, int COUT, int EPI>
