@@ -2626,14 +2626,29 @@ struct ListShared
 	uint32_t block[2];                    // colour and depth address of the sub-tile's first pixel
 };
 
-// The T threads that run a sub-tile together: thread 0 of them is aligned to T,
-// and `bar` is a barrier of their own (0 where they are the whole CTA).
-template <uint32_t T>
+// The T threads that run a sub-tile together, thread 0 of them aligned to T: the CTA
+// itself (GROUPS 0, barrier 0), or group k of GROUPS with barrier 1 + k of its own.
+// The barrier's number is part of the instruction: with one in a register a kernel is
+// taken to use all 16, and an SM has 64, for four CTAs, of 128 threads half of what its
+// registers hold (64 small streams in rounds 2.83 ms, so 2.14).  Not with eight groups
+// in 512 threads, where two CTAs fit anyway and choosing costs (AA1 streams 484 and 499 us).
+template <uint32_t T, uint32_t GROUPS = 0>
 struct ShadeGroup
 {
-	uint32_t bar;
+	uint32_t k;
 	__device__ __forceinline__ uint32_t thread() const { return threadIdx.x & (T - 1u); }
-	__device__ __forceinline__ void sync() const { asm volatile("bar.sync %0, %1;" ::"r"(bar), "n"(T) : "memory"); }
+	template <uint32_t B = 1>
+	__device__ __forceinline__ void sync() const
+	{
+		if constexpr (GROUPS == 0)
+			asm volatile("bar.sync 0, %0;" ::"n"(T) : "memory");
+		else if constexpr (T * GROUPS > 256u)
+			asm volatile("bar.sync %0, %1;" ::"r"(1u + k), "n"(T) : "memory");
+		else if (B == GROUPS || k + 1u == B)
+			asm volatile("bar.sync %0, %1;" ::"n"(B), "n"(T) : "memory");
+		else
+			sync<(B < GROUPS ? B + 1 : B)>();
+	}
 };
 
 template <uint32_t T, uint32_t CAP>
@@ -2646,7 +2661,8 @@ struct ListChunk
 	uint32_t total;
 
 	// Words [first, first + T * LIST_WORDS) of the `count` of the sub-tile.
-	__device__ __forceinline__ void load(const ShadeGroup<T> &G, const uint32_t *mask, uint32_t first, uint32_t count,
+	template <uint32_t GROUPS>
+	__device__ __forceinline__ void load(const ShadeGroup<T, GROUPS> &G, const uint32_t *mask, uint32_t first, uint32_t count,
 	                                     ListShared<T, CAP> &L)
 	{
 		const unsigned full = 0xffffffffu;
@@ -2676,7 +2692,8 @@ struct ListChunk
 	}
 
 	// Indices [round, round + CAP) of the chunk.
-	__device__ __forceinline__ void write(const ShadeGroup<T> &G, uint32_t prim_lo, uint32_t first, uint32_t round,
+	template <uint32_t GROUPS>
+	__device__ __forceinline__ void write(const ShadeGroup<T, GROUPS> &G, uint32_t prim_lo, uint32_t first, uint32_t round,
 	                                      ListShared<T, CAP> &L) const
 	{
 		#pragma unroll
@@ -2696,8 +2713,8 @@ struct ListChunk
 // the same sequence of covering primitives as walking the whole list.
 // `chunk` is the list's first chunk, loaded by the caller; with `written`, it is
 // the whole list and lies in L already.  RELOAD: the caller kept only its length.
-template <int NS, bool SS, bool AA, bool MIP, bool RELOAD, uint32_t T, uint32_t CAP>
-__device__ __forceinline__ void walk_list(const ShadeCtx &C, const DevInstance &I, const ShadeGroup<T> &G, const uint32_t *mask,
+template <int NS, bool SS, bool AA, bool MIP, bool RELOAD, uint32_t T, uint32_t CAP, uint32_t GROUPS>
+__device__ __forceinline__ void walk_list(const ShadeCtx &C, const DevInstance &I, const ShadeGroup<T, GROUPS> &G, const uint32_t *mask,
                                           ListChunk<T, CAP> &chunk, bool written, ListShared<T, CAP> &L, uint32_t t,
                                           SampleState &S, uint32_t &covered)
 {
@@ -2855,8 +2872,8 @@ __device__ __forceinline__ bool split_part(const PassParams &P, const DevInstanc
 }
 
 // Samples t of the sub-tile at (sub_x, sub_y), one per thread of the group.
-template <int NS, bool SS, bool AA, bool MIP, bool RELOAD, uint32_t T, uint32_t CAP>
-__device__ __forceinline__ void shade_part(const PassParams &P, const DevInstance &I, const ShadeGroup<T> &G, const uint32_t *mask,
+template <int NS, bool SS, bool AA, bool MIP, bool RELOAD, uint32_t T, uint32_t CAP, uint32_t GROUPS>
+__device__ __forceinline__ void shade_part(const PassParams &P, const DevInstance &I, const ShadeGroup<T, GROUPS> &G, const uint32_t *mask,
                                            int32_t sub_x, int32_t sub_y, ListChunk<T, CAP> &chunk, bool written, uint32_t t,
                                            ListShared<T, CAP> &list)
 {
@@ -3089,8 +3106,8 @@ __device__ __forceinline__ void shade_part(const PassParams &P, const DevInstanc
 // 2.18 ms.  Planes 0 and 1 alone give 1.70 and 2.72 ms.
 // fb and zb: swizzled index of the sub-tile's first pixel, which has to lie on the
 // 8-pixel grid for the sub-tile to be (part of) one block; nothing is asked for otherwise.
-template <int NS, uint32_t T>
-__device__ __forceinline__ void prefetch_planes(const PassParams &P, const DevInstance &I, const ShadeGroup<T> &G, uint32_t fb,
+template <int NS, uint32_t T, uint32_t GROUPS>
+__device__ __forceinline__ void prefetch_planes(const PassParams &P, const DevInstance &I, const ShadeGroup<T, GROUPS> &G, uint32_t fb,
                                                 uint32_t zb)
 {
 	if ((I.base_x | I.base_y) & 7)
@@ -3110,8 +3127,8 @@ __device__ __forceinline__ void prefetch_planes(const PassParams &P, const DevIn
 // One sub-tile's pixel samples, NS per pixel, one thread per sample: the T
 // threads of the group have samples t (of 64 * NS) and, with PARTS, the samples T,
 // 2 T ... further on.  SS selects the super-sampled path.
-template <int NS, bool SS, bool AA, bool MIP, uint32_t PARTS, uint32_t T, uint32_t CAP>
-__device__ __forceinline__ void shade_subtile(const PassParams &P, const DevInstance &I, const ShadeGroup<T> &G,
+template <int NS, bool SS, bool AA, bool MIP, uint32_t PARTS, uint32_t T, uint32_t CAP, uint32_t GROUPS>
+__device__ __forceinline__ void shade_subtile(const PassParams &P, const DevInstance &I, const ShadeGroup<T, GROUPS> &G,
                                               const uint32_t *sub_masks, uint32_t sub, uint32_t t, ListShared<T, CAP> &list)
 {
 	const uint32_t gx = sub % I.sub_w, gy = sub / I.sub_w;
@@ -3220,11 +3237,11 @@ constexpr uint32_t BATCH_MAX_NS_LOG2 = 2;
 
 // Separate functions per variant keep each variant's register allocation
 // its own inside the batched kernel.
-template <int NS, bool SS, bool AA, uint32_t T>
+template <int NS, bool SS, bool AA, uint32_t T, uint32_t BLOCK>
 __device__ __noinline__ void shade_subtile_call(const PassParams &P, const DevInstance &I, const uint32_t *sub_masks, uint32_t sub,
-                                                uint32_t t, uint32_t bar, ListShared<T, BATCH_LIST_CAP> &list)
+                                                uint32_t t, ListShared<T, BATCH_LIST_CAP> &list)
 {
-	shade_subtile<NS, SS, AA, false, 1, T, BATCH_LIST_CAP>(P, I, ShadeGroup<T>{ bar }, sub_masks, sub, t, list);
+	shade_subtile<NS, SS, AA, false, 1, T, BATCH_LIST_CAP>(P, I, ShadeGroup<T, BLOCK / T>{ threadIdx.x / T }, sub_masks, sub, t, list);
 }
 
 template <int BLOCK>
@@ -3281,7 +3298,7 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) batch_shade_kernel(const 
 		const uint32_t sub = sample >> (6u + it.ns_log2), t = sample & ((64u << it.ns_log2) - 1u);
 		const uint32_t mode = sub < I.sub_w * I.sub_h ? tile_mode(I, subtile_flags(P, I, it.flags, sub)) : 0u;
 		const uint32_t ns_log2 = mode == 2 ? it.ns_log2 : 0u;
-		// A group's barrier and list are those of its first 64 threads.
+		// A group's list lies in the slot of its first 64 threads.
 		if (mode && t < (64u << ns_log2))
 		{
 			const bool aa = it.aa != 0;
@@ -3289,21 +3306,21 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) batch_shade_kernel(const 
 			switch (ns_log2)
 			{
 			case 0:
-				if (aa) shade_subtile_call<1, false, true, T1>(P, I, it.masks, sub, t, 1u + s1, slots[s1].list);
-				else shade_subtile_call<1, false, false, T1>(P, I, it.masks, sub, t, 1u + s1, slots[s1].list);
+				if (aa) shade_subtile_call<1, false, true, T1, BLOCK>(P, I, it.masks, sub, t, slots[s1].list);
+				else shade_subtile_call<1, false, false, T1, BLOCK>(P, I, it.masks, sub, t, slots[s1].list);
 				break;
 			case 1:
 			{
 				auto &list = reinterpret_cast<ListShared<T2, BATCH_LIST_CAP> &>(slots[s2]);
-				if (aa) shade_subtile_call<2, true, true, T2>(P, I, it.masks, sub, t, 1u + s2, list);
-				else shade_subtile_call<2, true, false, T2>(P, I, it.masks, sub, t, 1u + s2, list);
+				if (aa) shade_subtile_call<2, true, true, T2, BLOCK>(P, I, it.masks, sub, t, list);
+				else shade_subtile_call<2, true, false, T2, BLOCK>(P, I, it.masks, sub, t, list);
 				break;
 			}
 			default:
 			{
 				auto &list = reinterpret_cast<ListShared<T4, BATCH_LIST_CAP> &>(slots[s4]);
-				if (aa) shade_subtile_call<4, true, true, T4>(P, I, it.masks, sub, t, 1u + s4, list);
-				else shade_subtile_call<4, true, false, T4>(P, I, it.masks, sub, t, 1u + s4, list);
+				if (aa) shade_subtile_call<4, true, true, T4, BLOCK>(P, I, it.masks, sub, t, list);
+				else shade_subtile_call<4, true, false, T4, BLOCK>(P, I, it.masks, sub, t, list);
 				break;
 			}
 			}
