@@ -1242,7 +1242,7 @@ struct CudaBackend
 				c.src_vram = d_snapshot;
 			}
 			StageScope ts(this, PGS_TIMESTAMP_COPY_VRAM);
-			upload_kernel<<<dim3((c.width + 31) / 32, (c.height + 7) / 8), 256, 0, stream>>>(c, d_vram);
+			upload_kernel<<<dim3(pixel_tiles_x(c), pixel_tiles_y(c)), 256, 0, stream>>>(c, d_vram);
 			launch_counter++;
 			CUDA_TRY(cudaGetLastError());
 			return PGS_OK;
@@ -1338,7 +1338,7 @@ struct CudaBackend
 				c.host = d_arena + list[j].copy_host_off;
 				B.c[B.count] = c;
 				B.block_start[B.count] = blocks;
-				blocks += upload_tiles_x(c) * upload_tiles_y(c);
+				blocks += upload_tiles(c);
 				B.count++;
 				j++;
 			}

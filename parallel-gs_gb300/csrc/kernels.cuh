@@ -3629,8 +3629,8 @@ __device__ __forceinline__ uint32_t read_pixel(const uint8_t *vram, uint32_t psm
 
 // One pixel of a transfer.  A single transfer's launch is its latency (eight 16x16
 // uploads of one place, in turn: 20 us), so it takes the shortest code: four pixels
-// per thread, as in the batched uploads below, made them 25 to 29 us, and eight
-// 256x256 local copies 45 to 55 us instead of 35 to 41.
+// per thread in all formats made them 25 to 29 us, and eight 256x256 local copies 45
+// to 55 us instead of 35 to 41.
 __device__ __forceinline__ void upload_pixel(const CopyParams &C, uint8_t *vram, uint32_t x, uint32_t y)
 {
 	if (x >= C.width || y >= C.height)
@@ -3672,22 +3672,31 @@ __device__ __forceinline__ void upload_pixel(const CopyParams &C, uint8_t *vram,
 	write_pixel(vram, C.dpsm, swizzle_address(dx, dy, C.dbp, C.dbw, C.dpsm), data, C.invalidate_ss != 0);
 }
 
-__global__ void __launch_bounds__(256) upload_kernel(CopyParams C, uint8_t *vram)
+// Pixels of the 32 x 8 tile at (tx, ty), one per thread.
+__host__ __device__ inline uint32_t pixel_tiles_x(const CopyParams &C) { return (C.width + 31u) / 32u; }
+__host__ __device__ inline uint32_t pixel_tiles_y(const CopyParams &C) { return (C.height + 7u) / 8u; }
+
+__device__ __forceinline__ void upload_tile(const CopyParams &C, uint8_t *vram, uint32_t tx, uint32_t ty)
 {
-	upload_pixel(C, vram, blockIdx.x * 32u + (threadIdx.x & 31u), blockIdx.y * 8u + (threadIdx.x >> 5));
+	upload_pixel(C, vram, tx * 32u + (threadIdx.x & 31u), ty * 8u + (threadIdx.x >> 5));
 }
 
-// Batched uploads go in tiles of 32 x 32 pixels from a multiple of 4 in the
-// destination on, a thread per four pixels of a row, which share one destination
-// address computation and, where they are aligned and all there, one payload load.
-// Bound: issue of the address arithmetic (eight 256x256 PSMT8 textures with their
-// palettes: a pixel per thread 4.7 M warp instructions, so 1.8; a light frame that
-// uploads them 24.5 -> 22.9 us per replay).
-__host__ __device__ inline uint32_t upload_tiles_x(const CopyParams &C) { return ((C.dsax & 3u) + C.width + 31u) / 32u; }
-__host__ __device__ inline uint32_t upload_tiles_y(const CopyParams &C) { return (C.height + 31u) / 32u; }
+__global__ void __launch_bounds__(256) upload_kernel(CopyParams C, uint8_t *vram)
+{
+	upload_tile(C, vram, blockIdx.x, blockIdx.y);
+}
 
-// Four pixels of the tile at (tx, ty) of a host->local upload.
-__device__ __forceinline__ void upload_quad(const CopyParams &C, uint8_t *vram, uint32_t tx, uint32_t ty)
+// Four pixels of the 32 x 32 tile at (tx, ty) of a PSMT8 upload per thread, from a
+// multiple of 4 in the destination on: they share one address computation and, where
+// they are aligned and all there, one payload load.  For the one format, the code is
+// short.  Bound: issue of the address arithmetic and latency (four launches of sixteen
+// 128x128 PSMT8 uploads 20.5 us with a pixel per thread, 16.1 so; light frame that
+// uploads eight 256x256 textures 24.5 and 22.4).  With all formats the longer code
+// made most batches slower (sixteen of PSMT4 22.6 -> 33, of PSMCT24 22.5 -> 28).
+__host__ __device__ inline uint32_t quad_tiles_x(const CopyParams &C) { return ((C.dsax & 3u) + C.width + 31u) / 32u; }
+__host__ __device__ inline uint32_t quad_tiles_y(const CopyParams &C) { return (C.height + 31u) / 32u; }
+
+__device__ __forceinline__ void upload_quad_tile(const CopyParams &C, uint8_t *vram, uint32_t tx, uint32_t ty)
 {
 	// Pixel k of the quad is column x0 + k of the rectangle (x0 may be negative).
 	const int32_t x0 = int32_t(tx * 32u + (threadIdx.x & 7u) * 4u) - int32_t(C.dsax & 3u);
@@ -3695,28 +3704,18 @@ __device__ __forceinline__ void upload_quad(const CopyParams &C, uint8_t *vram, 
 	if (y >= C.height || x0 >= int32_t(C.width))
 		return;
 	uint32_t limit = C.width;
-	{
-		// Columns past the buffer's stride are only written on the last page row.
-		uint32_t eff_stride = C.dbw;
-		if (C.dpsm == PSMT4 || C.dpsm == PSMT8)
-			eff_stride &= ~1u;
-		const Layout L = psm_layout(C.dpsm);
-		if ((C.dsay + C.height - 1u) >> L.ph != (C.dsay + y) >> L.ph)
-			limit = min(limit, eff_stride * 64u);
-	}
-	const uint32_t dx = uint32_t(x0 + int32_t(C.dsax)) & 2047u, dy = (y + C.dsay) & 2047u;
-	uint32_t data[4];
+	// Columns past the buffer's stride are only written on the last page row.
+	const Layout L = psm_layout(PSMT8);
+	if ((C.dsay + C.height - 1u) >> L.ph != (C.dsay + y) >> L.ph)
+		limit = min(limit, (C.dbw & ~1u) * 64u);
 	uint32_t have = 0; // pixels to write
-	const uint32_t b = psm_bits_per_pixel(C.dpsm);
-	const uint32_t factor = (b == 32 || b == 24) ? 2 : (b == 16 ? 4 : (b == 8 ? 8 : 16));
-	const uint64_t avail = b == 32 ? C.host_size / 4 : (b == 24 ? C.host_size / 3 : (b == 16 ? C.host_size / 2 : (b == 8 ? C.host_size : 2 * C.host_size)));
 	const uint32_t row = y * C.width;
 	#pragma unroll
 	for (int k = 0; k < 4; k++)
 	{
 		const int32_t x = x0 + k;
 		const uint64_t sa = uint64_t(row) + uint32_t(x);
-		if (x >= 0 && uint32_t(x) < limit && sa * factor >= C.host_offset_qwords && sa < avail)
+		if (x >= 0 && uint32_t(x) < limit && sa * 8u >= C.host_offset_qwords && sa < C.host_size)
 			have |= 1u << k;
 	}
 	if (!have)
@@ -3724,44 +3723,26 @@ __device__ __forceinline__ void upload_quad(const CopyParams &C, uint8_t *vram, 
 	// The payload starts 256-byte aligned.
 	const uint8_t *h = C.host;
 	const uint32_t sa = row + uint32_t(x0); // of pixel 0, if it is there
-	if (have == 15u && !(sa & 3u) && (b == 32 || b == 16 || b == 8))
-	{
-		if (b == 32)
-		{
-			const uint4 v = *reinterpret_cast<const uint4 *>(h + size_t(sa) * 4u);
-			data[0] = v.x; data[1] = v.y; data[2] = v.z; data[3] = v.w;
-		}
-		else if (b == 16)
-		{
-			const uint2 v = *reinterpret_cast<const uint2 *>(h + size_t(sa) * 2u);
-			data[0] = v.x & 0xffffu; data[1] = v.x >> 16; data[2] = v.y & 0xffffu; data[3] = v.y >> 16;
-		}
-		else
-		{
-			const uint32_t v = *reinterpret_cast<const uint32_t *>(h + sa);
-			data[0] = v & 0xffu; data[1] = (v >> 8) & 0xffu; data[2] = (v >> 16) & 0xffu; data[3] = v >> 24;
-		}
-	}
+	uint32_t data = 0;
+	if (have == 15u && !(sa & 3u))
+		data = *reinterpret_cast<const uint32_t *>(h + sa);
 	else
 	{
 		#pragma unroll
 		for (int k = 0; k < 4; k++)
-		{
-			if (!((have >> k) & 1u))
-				continue;
-			const size_t p = size_t(row) + uint32_t(x0 + k);
-			if (b == 24) data[k] = uint32_t(h[3 * p]) | (uint32_t(h[3 * p + 1]) << 8) | (uint32_t(h[3 * p + 2]) << 16);
-			else if (b == 16) data[k] = reinterpret_cast<const uint16_t *>(h)[p];
-			else if (b == 8) data[k] = h[p];
-			else if (b == 4) data[k] = (uint32_t(h[p >> 1]) >> ((p & 1) * 4)) & 15u;
-			else data[k] = reinterpret_cast<const uint32_t *>(h)[p];
-		}
+			if ((have >> k) & 1u)
+				data |= uint32_t(h[size_t(row) + uint32_t(x0 + k)]) << (8 * k);
 	}
-	const uint32_t a = swizzle_address(dx, dy, C.dbp, C.dbw, C.dpsm);
+	const uint32_t a = swizzle_address(uint32_t(x0 + int32_t(C.dsax)) & 2047u, (y + C.dsay) & 2047u, C.dbp, C.dbw, PSMT8);
 	#pragma unroll
 	for (int k = 0; k < 4; k++)
 		if ((have >> k) & 1u)
-			write_pixel(vram, C.dpsm, a + quad_offset(C.dpsm, uint32_t(k)), data[k], C.invalidate_ss != 0);
+			write_pixel(vram, PSMT8, a + quad_offset(PSMT8, uint32_t(k)), data >> (8 * k), C.invalidate_ss != 0);
+}
+
+__host__ __device__ inline uint32_t upload_tiles(const CopyParams &C)
+{
+	return C.dpsm == PSMT8 ? quad_tiles_x(C) * quad_tiles_y(C) : pixel_tiles_x(C) * pixel_tiles_y(C);
 }
 
 // Consecutive host->local uploads whose destination blocks do not overlap, in
@@ -3781,8 +3762,12 @@ __global__ void __launch_bounds__(256) upload_batch_kernel(UploadBatch B, uint8_
 	while (i + 1u < B.count && blockIdx.x >= B.block_start[i + 1])
 		i++;
 	const CopyParams &C = B.c[i];
-	const uint32_t local = blockIdx.x - B.block_start[i], tiles_x = upload_tiles_x(C);
-	upload_quad(C, vram, local % tiles_x, local / tiles_x);
+	const uint32_t local = blockIdx.x - B.block_start[i];
+	const uint32_t tiles_x = C.dpsm == PSMT8 ? quad_tiles_x(C) : pixel_tiles_x(C);
+	if (C.dpsm == PSMT8)
+		upload_quad_tile(C, vram, local % tiles_x, local / tiles_x);
+	else
+		upload_tile(C, vram, local % tiles_x, local / tiles_x);
 }
 
 // LOCAL->HOST read-out of a rectangle of plane 0 into linear bytes
