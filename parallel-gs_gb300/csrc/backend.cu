@@ -1154,14 +1154,19 @@ struct CudaBackend
 		// Super-sampled shading touches planes 1 .. 1 + 2^ns_log2.
 		if (I.rate_y_log2 != 0 && 2u + (1u << ns_log2) > num_planes)
 			return PGS_ERROR_INVALID_ARGUMENT;
-		// 8x and 16x: coarse tiles from this many primitives on have their sub-tiles
-		// split (ShadeCta).  Blended triangles in one sub-tile at 16x in turn and in
-		// CTAs of 1024 threads, which hold it whole: 300 0.39 and 0.67 ms, 2,000 2.41
-		// and 1.99; AA1 triangles 300 0.55 and 0.67, 2,000 3.15 and 1.88.  Not where
-		// tiles like it, if the pass consists of them, fill the GPU anyway: 20,000
-		// sprites all over the frame at 16x 676 us, with a CTA per part 695.
+		// 8x and 16x: all sub-tiles are split (ShadeCta) where their parts fit the GPU at
+		// once (one triangle at 16x through the live path 66 us in turn, 56 split; 1,000 in
+		// 16x16 pixels 206 and 126), at 8x from some primitives on (one triangle's replay
+		// 41.8 us, split 45.4; 100 in 16x16 pixels live 69 and 67, 1,000 145 and 123).
+		// Beyond, those of coarse tiles from this many primitives on.  Blended triangles in
+		// one sub-tile at 16x in turn and in CTAs of 1024 threads, which hold it whole: 300
+		// 0.39 and 0.67 ms, 2,000 2.41 and 1.99; AA1 triangles 300 0.55 and 0.67, 2,000
+		// 3.15 and 1.88.  Not where tiles like it, if the pass consists of them, fill the
+		// GPU anyway: 20,000 sprites all over the frame at 16x 676 us, a CTA per part 695.
 		const uint32_t from = p.has_aa1 || p.has_mipmap || p.has_ss_textures ? 256u : 1024u;
-		if (ns_log2 > 2 && count >= from)
+		if (ns_log2 > 2 && subs << (ns_log2 - 2u) <= shade_slots() && (ns_log2 > 3 || count >= 32u))
+			I.split_count = SPLIT_ALL;
+		else if (ns_log2 > 2 && count >= from)
 			I.split_count = std::max(from, uint32_t((uint64_t(count) << (2u * (p.tile_size_log2 - 3u))) / shade_slots()));
 		size_t mask_words = subs * I.mask_words;
 		// Sub-tile masks and the coarse tiles' flags, cleared together.

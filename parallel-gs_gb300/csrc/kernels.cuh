@@ -211,6 +211,7 @@ constexpr uint32_t TILE_HAS_ZW = 1u << 3;
 // Primitives binned to the tile, counted from this bit for blend demotion, or by
 // every eighth primitive for splitting.
 constexpr uint32_t TILE_COUNT_SHIFT = 8;
+constexpr uint32_t SPLIT_ALL = ~0u; // DevInstance::split_count: every tile
 
 constexpr uint32_t ERROR_FLAG_TILE_OVERFLOW = 1u << 0;
 
@@ -2829,7 +2830,7 @@ __device__ __forceinline__ uint32_t subtile_flags(const PassParams &P, const Dev
 // (ShadeCta).  Which CTA shades a part changes no result.
 __device__ __forceinline__ bool split_tile(const DevInstance &I, uint32_t flags)
 {
-	return I.split_count && (flags >> TILE_COUNT_SHIFT) >= I.split_count;
+	return I.split_count && ((flags >> TILE_COUNT_SHIFT) >= I.split_count || I.split_count == SPLIT_ALL);
 }
 
 // Part number `item` of all parts of the sub-tiles of split super-sampled tiles:

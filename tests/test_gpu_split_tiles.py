@@ -1,8 +1,9 @@
 """Sub-tiles whose parts go to CTAs of their own (8x and 16x) against the oracle:
 coarse tiles with a few primitives less and more than it takes, several of them,
 at the frame's corners and across tile borders, single-sampled ones among them,
-and tiles whose counts serve blend demotion too.  Which CTA shades a part changes
-no result: every plane and the covered-sample count must be equal."""
+and tiles whose counts serve blend demotion too; and instances small enough that
+all of them are split.  Which CTA shades a part changes no result: every plane and
+the covered-sample count must be equal."""
 import numpy as np
 import pytest
 
@@ -60,3 +61,19 @@ def test_clusters(ss, n, aa1):
 @pytest.mark.parametrize("ss", [8, 16])
 def test_clusters_with_blend_demotion(ss):
     assert_same(*run_both(frame(ss, 1100, 0, blended=True, hacks={"allow_blend_demote": True})))
+
+
+@pytest.mark.parametrize("ss", [8, 16])
+@pytest.mark.parametrize("w,h", [(8, 8), (33, 17), (96, 96), (104, 96), (152, 128), (160, 128)])
+@pytest.mark.parametrize("n,aa1", [(5, 0), (28, 0), (29, 0), (300, 0), (60, 1)])
+def test_small_instances(ss, w, h, n, aa1):
+    """Up to 152 sub-tiles at 16x, and 304 at 8x from 32 primitives on, are all split."""
+    rng = np.random.default_rng(ss * w + n)
+    s = gsgen.GifStream()
+    gsgen._frame_setup(s, 0, W // 64, gsgen.PSMCT32, ZBP, gsgen.PSMZ24, W, H, gsgen.test_reg(zte=1, ztst=2),
+                       alpha=gsgen.alpha_reg(0, 1, 0, 1), extra=[(gsgen.COLCLAMP, 1)])
+    s.ad([(gsgen.SCISSOR_1, gsgen.scissor_reg(24, 24 + w - 1, 40, 40 + h - 1))])
+    flat_sprites(s, rng, 1, 24, 40)
+    cluster(s, rng, n, 20, 36, max(w, h) + 8, aa1=aa1)
+    cluster(s, rng, 2, 20, 36, max(w, h) + 8, abe=1)
+    assert_same(*run_both(gsgen.Frame("small", s.tobytes(), ss, ss == 16, n + 3, {"width": W, "height": H})))
