@@ -1178,7 +1178,8 @@ struct CudaBackend
 			StageScope ts(this, PGS_TIMESTAMP_BINNING);
 			CUDA_TRY(cudaMemsetAsync(d_masks, 0, (mask_words + tiles) * sizeof(uint32_t), stream));
 			// A pass of few primitives spreads each group's candidates over more CTAs.
-			const uint32_t groups = (count + 31) / 32, slices = std::min(std::max(BIN_TARGET_CTAS / groups, 1u), 16u);
+			const uint32_t groups = (count + 31) / 32;
+			const uint32_t slices = std::min(std::max(uint32_t(sm_count) * BIN_CTAS_PER_SM / groups, 1u), 16u);
 			bin_kernel<<<dim3(groups, slices), 32 * BIN_GROUP_WARPS, 0, stream>>>(P, I, d_masks, d_flags);
 			launch_counter++;
 		}

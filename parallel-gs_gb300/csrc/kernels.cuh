@@ -997,8 +997,8 @@ __device__ __forceinline__ bool intersects_tile(const PrimSetup &s, int32_t lo0,
 // of its primitive and one CTA per group, a 61-primitive frame with a clear of
 // the whole frame took 47 us here and takes 4; a feedback frame's passes at 8x went from 15 to 4.6.
 constexpr uint32_t BIN_GROUP_WARPS = 4;
-// CTAs a launch aims at when its groups are fewer (four per SM), up to 16 per group.
-constexpr uint32_t BIN_TARGET_CTAS = 608;
+// CTAs per SM that a launch aims at when its groups are fewer, up to 16 CTAs per group.
+constexpr uint32_t BIN_CTAS_PER_SM = 4;
 
 // One live primitive of a group, as the dealt-out tests read it.
 struct BinItem
