@@ -1095,7 +1095,7 @@ struct CudaBackend
 	{
 		if (I.rate_y_log2 != 0)
 		{
-			// Behind the sub-tiles' CTAs those for the parts of split ones, as many as fit the GPU.
+			// With the sub-tiles' CTAs those for the parts of split ones, as many as fit the GPU.
 			const uint32_t more = I.split_count ? std::min(shade_slots(), grid << (ns_log2 - 2u)) : 0u;
 			switch (ns_log2)
 			{
@@ -1168,6 +1168,8 @@ struct CudaBackend
 			I.split_count = SPLIT_ALL;
 		else if (ns_log2 > 2 && count >= from)
 			I.split_count = std::max(from, uint32_t((uint64_t(count) << (2u * (p.tile_size_log2 - 3u))) / shade_slots()));
+		if (I.split_count)
+			I.split_first = std::min(uint32_t(sm_count), uint32_t(subs) << (ns_log2 - 2u));
 		size_t mask_words = subs * I.mask_words;
 		// Sub-tile masks and the coarse tiles' flags, cleared together.
 		int r = ensure_masks(mask_words + tiles);

@@ -71,6 +71,7 @@ struct DevInstance
 	uint32_t force_ss;            // field rendering: every covered tile super-sampled
 	uint32_t blend_demote;        // primitives per coarse tile that demote a blended tile, 0 = off
 	uint32_t split_count;         // primitives per coarse tile that split its sub-tiles (split_tile), 0 = never
+	uint32_t split_first;         // CTAs for split parts in front of those of the sub-tiles
 };
 
 // Linear RGBA8 image decoded from swizzled VRAM + CLUT for one mip level of
@@ -2594,9 +2595,12 @@ __device__ __forceinline__ void walk_batch(const ShadeCtx &C, const uint32_t *id
 // 2.48 ms whole, 1.93 a CTA per part, 1.72 so; at 16x 5.07, 3.51, 2.74).
 // A long list is the launch's critical path, though, and the parts in turn make it
 // as many times longer, so the sub-tiles of coarse tiles with many primitives are
-// split: CTAs behind those of the sub-tiles take their parts (2,000 blended
-// triangles in one sub-tile at 16x 2.41 -> 0.77 ms, 36,000 AA1 triangles within
-// 64x64 pixels 2.13 -> 0.67).  Which tiles: run_instance.
+// split.  Their parts are taken by CTAs in front of those of the sub-tiles, one per SM,
+// so that a long list starts with the launch (3,000 primitives in 16x16 pixels next to
+// 4,000 all over a 1024x900 frame at 8x: 440 us in turn, 441 split with all such CTAs
+// behind, 291 so), and by more behind (2,000 blended triangles in one sub-tile at 16x
+// 2.41 -> 0.77 ms, 36,000 AA1 triangles within 64x64 pixels 2.13 -> 0.68).  Which tiles:
+// run_instance.
 template <int NS>
 struct ShadeCta
 {
@@ -2839,35 +2843,43 @@ template <uint32_t PARTS, uint32_t T, uint32_t CAP>
 __device__ __forceinline__ bool split_part(const PassParams &P, const DevInstance &I, const uint32_t *tile_flags, uint32_t item,
                                            const ShadeGroup<T> &G, ListShared<T, CAP> &list, uint32_t &sub, uint32_t &part)
 {
+	constexpr uint32_t WARPS = T / 32u;
+	static_assert(LIST_WORDS * WARPS == 32u, "one count per lane");
+	const unsigned full = 0xffffffffu;
 	const uint32_t sh = P.tile_size_log2 - 3u, per_tile = PARTS << (2u * sh);
 	const uint32_t want = item / per_tile, k = item % per_tile; // tile by rank, part in it
 	const uint32_t lane = G.thread() & 31u, warp = G.thread() >> 5, tiles = I.tiles_w * I.tiles_h;
 	uint32_t seen = 0;
-	for (uint32_t base = 0; base < tiles; base += T)
+	for (uint32_t base = 0; base < tiles; base += T * LIST_WORDS)
 	{
-		const uint32_t tile = base + G.thread(), flags = tile < tiles ? tile_flags[tile] : 0u;
-		const bool split = tile_mode(I, flags) == 2u && split_tile(I, flags);
-		const uint32_t m = __ballot_sync(0xffffffffu, split);
-		if (lane == 0)
-			list.count[warp] = uint32_t(__popc(m));
-		G.sync();
-		uint32_t rank = seen + uint32_t(__popc(m & ((1u << lane) - 1u)));
-		for (uint32_t w = 0; w < T / 32u; w++)
+		uint32_t split[LIST_WORDS]; // of the warp's tiles
+		#pragma unroll
+		for (uint32_t q = 0; q < LIST_WORDS; q++)
 		{
-			const uint32_t c = list.count[w];
-			rank += w < warp ? c : 0u;
-			seen += c;
+			const uint32_t tile = base + q * T + G.thread(), flags = tile < tiles ? tile_flags[tile] : 0u;
+			split[q] = __ballot_sync(full, tile_mode(I, flags) == 2u && split_tile(I, flags));
+			if (lane == 0)
+				list.count[q * WARPS + warp] = uint32_t(__popc(split[q]));
 		}
-		if (split && rank == want)
-			list.ids[0] = tile;
 		G.sync();
-		if (want < seen)
+		const uint32_t v = list.count[lane], x = warp_scan(v, lane), total = __shfl_sync(full, x, 31);
+		if (want - seen < total)
 		{
+			#pragma unroll
+			for (uint32_t q = 0; q < LIST_WORDS; q++)
+			{
+				const uint32_t before = seen + __shfl_sync(full, x - v, int(q * WARPS + warp));
+				if (((split[q] >> lane) & 1u) && before + uint32_t(__popc(split[q] & ((1u << lane) - 1u))) == want)
+					list.ids[0] = base + q * T + G.thread();
+			}
+			G.sync();
 			const uint32_t t = list.ids[0], in = k / PARTS;
 			sub = ((t / I.tiles_w << sh) + (in >> sh)) * I.sub_w + (t % I.tiles_w << sh) + (in & ((1u << sh) - 1u));
 			part = k % PARTS;
 			return true;
 		}
+		seen += total;
+		G.sync();
 	}
 	return false;
 }
@@ -3190,10 +3202,9 @@ __global__ void __launch_bounds__(ShadeCta<NS>::THREADS, PGS_SHADE_MIN_BLOCKS(NS
 	constexpr uint32_t T = ShadeCta<NS>::THREADS, PARTS = ShadeCta<NS>::PARTS;
 	__shared__ ListShared<T, SHADE_LIST_CAP> list;
 	const ShadeGroup<T> G{ 0u };
-	const uint32_t subs = I.sub_w * I.sub_h;
-	uint32_t sub = blockIdx.x;
+	uint32_t sub = blockIdx.x - (PARTS > 1 ? I.split_first : 0u);
 	// The usual case comes first: behind the other, each launch took 3 us longer.
-	if (sub < subs)
+	if (sub < I.sub_w * I.sub_h)
 	{
 		const uint32_t flags = subtile_flags(P, I, tile_flags, sub);
 		if (tile_mode(I, flags) == (SS ? 2u : 1u) && !(PARTS > 1 && split_tile(I, flags)))
@@ -3202,9 +3213,11 @@ __global__ void __launch_bounds__(ShadeCta<NS>::THREADS, PGS_SHADE_MIN_BLOCKS(NS
 	}
 	if constexpr (PARTS > 1)
 	{
-		// Parts of split sub-tiles, one after another.
-		uint32_t part;
-		for (uint32_t item = sub - subs; split_part<PARTS>(P, I, tile_flags, item, G, list, sub, part); item += gridDim.x - subs)
+		// Every so many-th part of split sub-tiles.  (A counter that hands them out evened
+		// the CTAs' loads a little, but the longer code cost all launches 4 us.)
+		const uint32_t subs = I.sub_w * I.sub_h;
+		uint32_t part, item = blockIdx.x < I.split_first ? blockIdx.x : blockIdx.x - subs;
+		for (; split_part<PARTS>(P, I, tile_flags, item, G, list, sub, part); item += gridDim.x - subs)
 		{
 			shade_subtile<NS, SS, AA, MIP, 1, T, SHADE_LIST_CAP>(P, I, G, sub_masks, sub, threadIdx.x + part * T, list);
 			__syncthreads();

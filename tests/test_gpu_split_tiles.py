@@ -77,3 +77,24 @@ def test_small_instances(ss, w, h, n, aa1):
     cluster(s, rng, n, 20, 36, max(w, h) + 8, aa1=aa1)
     cluster(s, rng, 2, 20, 36, max(w, h) + 8, abe=1)
     assert_same(*run_both(gsgen.Frame("small", s.tobytes(), ss, ss == 16, n + 3, {"width": W, "height": H})))
+
+
+@pytest.mark.parametrize("ss", [8, 16])
+def test_many_coarse_tiles(ss):
+    """1120 coarse tiles of 16x16 pixels: the split ones are found 1024 at a time."""
+    w, h = 640, 448
+    rng = np.random.default_rng(ss)
+    s = gsgen.GifStream()
+    gsgen._frame_setup(s, 0, w // 64, gsgen.PSMCT32, 140, gsgen.PSMZ24, w, h, gsgen.test_reg(zte=1, ztst=2),
+                       alpha=gsgen.alpha_reg(0, 1, 0, 1), extra=[(gsgen.COLCLAMP, 1)])
+    n, spots = 1100, ((0, 0), (632, 96), (320, 104), (8, 328), (632, 440))
+    x0, y0 = (np.repeat(np.array(spots)[:, k], n) for k in (0, 1))
+    x = x0[:, None] * 16 + rng.integers(0, 128, size=(n * len(spots), 3))
+    y = y0[:, None] * 16 + rng.integers(0, 128, size=(n * len(spots), 3))
+    q = np.zeros((x.size, 2, 2), dtype=np.uint64)
+    q[:, 0] = gsgen.q_rgbaq(rng.integers(0, 256, size=(x.size, 4), dtype=np.int64))
+    q[:, 1] = gsgen.q_xyz2(x.reshape(-1), y.reshape(-1), rng.integers(0, 1 << 24, size=x.size))
+    for k in range(len(spots)):
+        s.packed(gsgen.prim_reg(gsgen.PRIM_TRI, iip=1, abe=k & 1), [gsgen.D_RGBAQ, gsgen.D_XYZ2],
+                 q[k * 3 * n:(k + 1) * 3 * n].reshape(-1, 2))
+    assert_same(*run_both(gsgen.Frame("spots", s.tobytes(), ss, True, n * len(spots), {"width": w, "height": h})))
