@@ -81,11 +81,6 @@ __device__ __forceinline__ void ldsm_x2(uint32_t addr, uint32_t &r0, uint32_t &r
 	asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0,%1}, [%2];\n" : "=r"(r0), "=r"(r1) : "r"(addr));
 }
 
-__device__ __forceinline__ void ldsm_x2_t(uint32_t addr, uint32_t &r0, uint32_t &r1)
-{
-	asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0,%1}, [%2];\n" : "=r"(r0), "=r"(r1) : "r"(addr));
-}
-
 // D = A(16x16, row) * B(16x8, col) + D, BF16 in, FP32 accumulate.
 __device__ __forceinline__ void mma_bf16(float *d, const uint32_t *a, uint32_t b0, uint32_t b1)
 {
@@ -1314,12 +1309,12 @@ struct Upscaler
 		return PGS_OK;
 	}
 
-	// Forward pass of `n` images of h x w RGBA8 (device memory).  The FP32
-	// result stays in d_out; out_rgba (device, optional) gets it clamped and
-	// rounded to RGBA8.
-	// keep_input: the 16-channel BF16 input is kept in d_x0 (training needs
-	// it for the first layer's weight gradient); otherwise the first layer
-	// reads the RGBA8 image directly.
+	// Forward pass of `n` images of h x w RGBA8 (device memory).  out_rgba
+	// (device, optional) gets the result clamped and rounded to RGBA8.
+	// keep_input (training): the 16-channel BF16 input is kept in d_x0, for the
+	// first layer's weight gradient; otherwise the first layer reads the RGBA8
+	// image directly.  The FP32 result goes to d_out with keep_input or without
+	// out_rgba; else d_out keeps what it held.
 	int forward(const uint8_t *d_img, int n, int h, int w, uint8_t *out_rgba, bool keep_input)
 	{
 		size_t pixels = size_t(n) * h * w;
