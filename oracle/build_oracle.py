@@ -10,7 +10,7 @@ libpgsref_frontend.so
                gs/page_tracker.cpp, gs/gs_util.cpp) compiled unmodified over
                the recording renderer of ref_frontend/ref_frontend.cpp.
 The reference's sources are read where the reference is mounted:
-$PGS_REFERENCE_DIR, else /root/reference.  Where they are absent these two
+$PGS_REFERENCE_DIR, else reference_dir()'s default.  Where they are absent these two
 are not built and the tests that need them skip.
 
 Outputs go to oracle/_build and oracle/_ref (both git-ignored).

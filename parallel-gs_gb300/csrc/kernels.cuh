@@ -2346,13 +2346,13 @@ __device__ __forceinline__ bool depth_hidden(const ShadeCtx &C, const PrimSetup 
 // of covered samples, the depth bound, then in order the primitives that are
 // left.  zmin is taken once per call: depths only grow until a primitive writes
 // depth without a test, so a lane behind such a primitive keeps its primitive.
-// Bound: instruction issue (77 % of the issue slots, the integer pipe 70 % busy).
+// Bound: instruction issue (74 % of the issue slots, the integer pipe 62 % busy).
 // A lane per primitive evaluates 32 samples of 32 primitives in about 250
 // instructions where a lane per sample took about 70 per primitive, and on the
 // textured 640x448 frame with 52,000 primitives at 4x the depth bound drops
 // 3.2 M of the 4.4 M (primitive, warp) pairs that cover something; with the
 // single shading call below, which keeps the loop in the instruction cache,
-// the frame's shading went from 1.08 to 0.59 ms (1.12 G to 0.54 G warp
+// the frame's shading went from 1.08 to 0.53 ms (1.12 G to 0.47 G warp
 // instructions).  Plain 10,000-triangle frame at 1x: 70 to 47 us.
 // With few primitives in the batch (NS >= 4), two or four lanes share one and
 // take a part of its samples each.

@@ -365,8 +365,9 @@ __global__ void __launch_bounds__(256, EPI == EPI_LAST ? 8 : 4) conv3x3_kernel(C
 // and its dY are copied asynchronously into one of two buffers while the other
 // is multiplied.  A tile's 16 k16 steps are summed by the tensor cores, the
 // tiles' sums in FP32.
-// Bound: shared-memory reads of the fragments (about 2300 cycles a tile) next to
-// the legacy MMA's rate.  The version with a shared-memory sum that every warp
+// Bound: latency, with the legacy MMA pipe at 42 % of its cycles: the warps wait on
+// the fragments' shared-memory reads and on each tile's barriers, and the sums in
+// registers (96 a thread) and the two buffers (93 KB) leave 18 warps per SM.  The version with a shared-memory sum that every warp
 // added each tap of each tile to, and one thread per channel for the bias, took
 // 138 us for a 32 -> 32 layer of 16 128x128 crops; this takes 23 us.  The bias
 // goes to global memory once per CTA: once per warp and channel, on one cache
